@@ -465,10 +465,10 @@ int enqueue_delaunay_mult(tecs_sim* s, const PassArgs& a, int& K) {
   const unsigned L = launch_count(s);
   // applications per pair on this pass's positions, before the pass
   PROF_BEGIN(s);
-  if (s->d.dims == 3) k_delaunay_mult<3><<<L ? L : 1, kDelaunayThreads, 0, s->stream>>>(a.X, s->ctr, s->fp.rc2,
-                                                                                       s->d.capacity, s->dmult);
-  else k_delaunay_mult<2><<<L ? L : 1, kDelaunayThreads, 0, s->stream>>>(a.X, s->ctr, s->fp.rc2, s->d.capacity,
-                                                                           s->dmult);
+  const dim3 mb(L ? L : 1, kDelaunaySplit);
+  if (s->d.dims == 3) k_delaunay_mult<3><<<mb, kDelaunayThreads, 0, s->stream>>>(a.X, s->ctr, s->fp.rc2, s->d.capacity,
+                                                                                 s->dmult);
+  else k_delaunay_mult<2><<<mb, kDelaunayThreads, 0, s->stream>>>(a.X, s->ctr, s->fp.rc2, s->d.capacity, s->dmult);
   PROF_END(s, "k_delaunay_mult");
   K += 1;
   return 0;
