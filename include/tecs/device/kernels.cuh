@@ -902,9 +902,7 @@ __device__ __forceinline__ void visit(const GridP& g, const ForceP& fp, const Pa
   if (D >= 3) d2 = d2 + disp[2] * disp[2];
   if (d2 >= fp.rc2) return;
   if (FINDER == 3 && gabriel_blocked<D>(g, fp, a.X, a.off, i, j, xi, disp, d2)) return;
-  if (FINDER == 2 && gabriel_blocked_naive<D>(fp, a.X, n, i, j, xi, disp, d2)) return;
-  unsigned reps = FINDER == 5 ? reps5 : 1u;
-  if (FINDER == 4 && (reps = a.dmult[(size_t)i * a.capacity + j]) == 0u) return;
+  const unsigned reps = FINDER == 5 ? reps5 : 1u;
   if (a.pairs) {
     unsigned long long s = atomicAdd(&a.ctr->pair_count, (unsigned long long)reps);
     for (unsigned r = 0; r < reps; ++r)
@@ -1222,6 +1220,7 @@ static __global__ void __launch_bounds__(kPassThreads) k_pass(GridP g, ForceP fp
 template <int D, int FINDER, int FORCE>
 __device__ __forceinline__ void cell_general(const GridP& g, const ForceP& fp, const PassArgs& a, unsigned n, unsigned i,
                                           const float* xi, float2 pi, unsigned idi, Acc& acc) {
+    static_assert(FINDER == 1 || FINDER == 3 || FINDER == 5, "the naive finders run in k_pass_naive");
     if (FINDER == 1 || FINDER == 3) {
       int bc[3] = {0, 0, 0};
       if (FINDER == 1) bin_coords_mul<D>(g, xi, bc);
@@ -1245,19 +1244,164 @@ __device__ __forceinline__ void cell_general(const GridP& g, const ForceP& fp, c
           }
         }
       }
-    } else if (FINDER == 5) {
-      // the cell's Delaunay partners, ascending j, each applied reps times
+    } else {
+      // FINDER 5: the cell's Delaunay partners, ascending j, each applied reps times
       const unsigned m = a.dl_len[i];
       for (unsigned t = 0; t < m; ++t) {
         const uint2 e = a.dl_row[(size_t)i * kDlRow + t];
         visit<D, FINDER, FORCE>(g, fp, a, n, i, e.x, xi, pi, acc, idi, e.y);
       }
-    } else {
-      for (unsigned j = 0; j < n; ++j) {
-        if (j == i) continue;
-        visit<D, FINDER, FORCE>(g, fp, a, n, i, j, xi, pi, acc, idi);
+    }
+}
+
+// The naive finders' pass (FINDER 0, 2, 4: every j is a candidate), one warp
+// per CELLS cells: the lanes test 32 candidates at a time, the in-cutoff
+// lanes form their pairs' terms side by side, and the terms are added in j
+// order -- the reference's order, so the sums are those of cell_general bit
+// for bit.  A Gabriel pair's witnesses are tested by all lanes.
+// What bounds it: instruction issue and L1/L2 reads of the positions.  One
+// thread per cell (the form before) walks the n candidates in one dependent
+// chain and fills 21 of 152 SMs at 2,003 cells: 280 us a pass there.
+constexpr int kNaiveThreads = 256;
+
+template <int D, int FINDER, int FORCE, int CELLS>
+static __global__ void __launch_bounds__(kNaiveThreads) k_pass_naive(GridP g, ForceP fp, PassArgs a) {
+  static_assert(FINDER == 0 || FINDER == 2 || FINDER == 4, "the naive finders");
+  const unsigned n = a.ctr->n;
+  const unsigned lane = threadIdx.x & 31u;
+  const unsigned i0 = (blockIdx.x * (kNaiveThreads / 32) + (threadIdx.x >> 5)) * CELLS;
+  float xs[CELLS][3];
+  float2 ps[CELLS];
+  unsigned ids[CELLS];
+  Acc acc[CELLS];
+#pragma unroll
+  for (int c = 0; c < CELLS; ++c) {
+    const unsigned i = i0 + c;
+    const float4 v = i < n ? __ldg(&a.X[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    xs[c][0] = v.x; xs[c][1] = v.y; xs[c][2] = v.z;
+    ids[c] = id_of(v);
+    ps[c] = (FORCE == 2 && a.P && i < n) ? a.P[i] : make_float2(0.f, 0.f);
+    acc[c] = Acc{{0.f, 0.f, 0.f}, {0.f, 0.f}};
+  }
+  constexpr int U = 4;  // rounds of 32 candidates in flight
+  for (unsigned j0 = 0; j0 < (i0 < n ? n : 0u); j0 += 32u * U) {
+    float4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned j = j0 + 32u * u + lane;
+      v[u] = j < n ? __ldg(&a.X[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned j = j0 + 32u * u + lane;
+#pragma unroll
+      for (int c = 0; c < CELLS; ++c) {
+        const unsigned i = i0 + c;
+        float disp[3] = {xs[c][0] - v[u].x, xs[c][1] - v[u].y, 0.f};
+        float d2 = disp[0] * disp[0] + disp[1] * disp[1];
+        if (D >= 3) { disp[2] = xs[c][2] - v[u].z; d2 = d2 + disp[2] * disp[2]; }
+        bool in = j < n && j != i && i < n && !(d2 >= fp.rc2);
+        unsigned bits = __ballot_sync(0xffffffffu, in);
+        if (!bits) continue;
+        if (FINDER == 2) {
+          // one in-cutoff pair at a time: a witness in the ball around its midpoint
+          unsigned keep = 0u;
+          for (unsigned b = bits; b; b &= b - 1u) {
+            const int src = __ffs(b) - 1;
+            const unsigned jj = j0 + 32u * u + (unsigned)src;
+            float m[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+            for (int d = 0; d < D; ++d) m[d] = xs[c][d] - __shfl_sync(0xffffffffu, disp[d], src) * 0.5f;
+            const float rsq = __shfl_sync(0xffffffffu, d2, src) * 0.25f * fp.gab_csq;
+            bool blocked = false;
+            for (unsigned k0 = 0; k0 < n && !blocked; k0 += 64u) {
+              bool hit = false;
+#pragma unroll
+              for (int w = 0; w < 2; ++w) {
+                const unsigned k = k0 + 32u * w + lane;
+                if (k < n && k != i && k != jj) {
+                  const float4 q = __ldg(&a.X[k]);
+                  const float e0 = q.x - m[0], e1 = q.y - m[1];
+                  float s = e0 * e0 + e1 * e1;
+                  if (D >= 3) { const float e2 = q.z - m[2]; s = s + e2 * e2; }
+                  hit = hit || s < rsq;
+                }
+              }
+              blocked = __any_sync(0xffffffffu, hit);
+            }
+            if (!blocked) keep |= 1u << src;
+          }
+          bits = keep;
+          in = (keep >> lane) & 1u;
+        }
+        unsigned reps = 1u;
+        if (FINDER == 4) {
+          reps = in ? a.dmult[(size_t)i * a.capacity + j] : 0u;
+          in = reps != 0u;
+          bits = __ballot_sync(0xffffffffu, in);
+        }
+        if (!bits) continue;
+        float s[3] = {0.f, 0.f, 0.f}, bv[3], bp[2], al[2];
+        if (in) {
+          if (a.pairs) {
+            const unsigned long long at = atomicAdd(&a.ctr->pair_count, (unsigned long long)reps);
+            for (unsigned r = 0; r < reps; ++r)
+              if (at + r < a.pair_cap) a.pairs[at + r] = make_uint2(ids[c], id_of(v[u]));
+          }
+          const float dist = sqrtf(d2);
+          if (FORCE != 0) spring_term<D>(fp, disp, dist, s);
+          if (FORCE == 2) {
+            const float2 pj = a.P ? a.P[j] : make_float2(0.f, 0.f);
+            polarity_terms(fp, disp, dist, ps[c], pol_trig(ps[c]), pj, pol_trig(pj), bv, bp, al);
+          }
+        }
+        // a pair at distance zero has a +0 spring term, which leaves the sum unchanged
+        for (; bits && FORCE != 0; bits &= bits - 1u) {
+          const int src = __ffs(bits) - 1;
+          const unsigned rr = FINDER == 4 ? __shfl_sync(0xffffffffu, reps, src) : 1u;
+          float t[10];
+#pragma unroll
+          for (int d = 0; d < D; ++d) t[d] = __shfl_sync(0xffffffffu, s[d], src);
+          if (FORCE == 2) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) t[3 + d] = __shfl_sync(0xffffffffu, bv[d], src);
+#pragma unroll
+            for (int d = 0; d < 2; ++d) {
+              t[6 + d] = __shfl_sync(0xffffffffu, bp[d], src);
+              t[8 + d] = __shfl_sync(0xffffffffu, al[d], src);
+            }
+          }
+          for (unsigned r = 0; r < rr; ++r) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) acc[c].x[d] = acc[c].x[d] + t[d];
+            if (FORCE == 2) {
+#pragma unroll
+              for (int d = 0; d < 3; ++d) acc[c].x[d] = acc[c].x[d] + t[3 + d];
+              acc[c].p[0] = acc[c].p[0] + t[6];
+              acc[c].p[1] = acc[c].p[1] + t[7];
+              acc[c].p[0] = acc[c].p[0] + t[8];
+              acc[c].p[1] = acc[c].p[1] + t[9];
+            }
+          }
+        }
       }
     }
+  }
+  // lane c commits cell c
+  Acc mine = acc[0];
+  float2 pi = ps[0];
+#pragma unroll
+  for (int c = 1; c < CELLS; ++c)
+    if (lane == (unsigned)c) {
+      mine = acc[c];
+      pi = ps[c];
+    }
+  const unsigned i = i0 + lane;
+  const bool active = lane < (unsigned)CELLS && i < n;
+  const float4 vi = active ? a.X[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float xi[3] = {vi.x, vi.y, vi.z};
+  if (active && FORCE != 2 && a.P) pi = a.P[i];
+  pass_epilogue<D>(g, a, active, n, i, xi, vi, pi, mine);
 }
 
 // ---------------------------------------------------------------------------

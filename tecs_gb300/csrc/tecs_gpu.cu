@@ -285,6 +285,14 @@ bool coop_pass(const tecs_sim* s) {
   return s->d.finder == TECS_FINDER_BINNED_GABRIEL && geom && s->d.gabriel_coefficient <= 0.9f;
 }
 
+// The naive finders' pass: cells per warp.  One cell a warp fills the GPU up
+// to kNaiveOneCell cells; above, a warp takes four, which share each read of
+// the candidates' positions.
+constexpr unsigned kNaiveOneCell = 16384;
+unsigned naive_cells(const tecs_sim* s) {
+  return s->d.finder == TECS_FINDER_NAIVE_DELAUNAY || launch_count(s) <= kNaiveOneCell ? 1u : 4u;
+}
+
 PassFn pass_fn(const tecs_sim* s, bool sym) {
   const int D = s->d.dims, F = s->d.finder, FO = s->d.force;
   const bool coop_geom = coop_geometry(s);
@@ -307,15 +315,29 @@ PassFn pass_fn(const tecs_sim* s, bool sym) {
       if (DD == 3) return k_pass<DD, FF, 2>;                                    \
     }                                                                           \
   }
-  PICK(3, 0) PICK(3, 1) PICK(3, 2) PICK(3, 3) PICK(2, 0) PICK(2, 1) PICK(2, 2) PICK(2, 3)
+  PICK(3, 1) PICK(3, 3) PICK(2, 1) PICK(2, 3)
 #undef PICK
-  if (F == TECS_FINDER_NAIVE_DELAUNAY && !sym) {
-    if (D == 3 && FO == 0) return k_pass<3, 4, 0>;
-    if (D == 3 && FO == 1) return k_pass<3, 4, 1>;
-    if (D == 3 && FO == 2) return k_pass<3, 4, 2>;
-    if (D == 2 && FO == 0) return k_pass<2, 4, 0>;
-    if (D == 2 && FO == 1) return k_pass<2, 4, 1>;
+#define PICK_SYM(DD, FF)                                                        \
+  if (D == DD && F == FF && sym) {                                              \
+    if (FO == 0) return k_pass_sym<DD, FF, 0>;                                  \
+    if (FO == 1) return k_pass_sym<DD, FF, 1>;                                  \
+    if (DD == 3) return k_pass_sym<DD, FF, 2>;                                  \
   }
+  PICK_SYM(3, 0) PICK_SYM(3, 2) PICK_SYM(2, 0) PICK_SYM(2, 2)
+#undef PICK_SYM
+#define PICK_NAIVE(DD, FF, CC)                                                  \
+  if (D == DD && F == FF && !sym) {                                             \
+    if (FO == 0) return k_pass_naive<DD, FF, 0, CC>;                            \
+    if (FO == 1) return k_pass_naive<DD, FF, 1, CC>;                            \
+    if (DD == 3) return k_pass_naive<3, FF, 2, CC>;                             \
+  }
+  if (naive_cells(s) == 1) {
+    PICK_NAIVE(3, 0, 1) PICK_NAIVE(3, 2, 1) PICK_NAIVE(3, 4, 1)
+    PICK_NAIVE(2, 0, 1) PICK_NAIVE(2, 2, 1) PICK_NAIVE(2, 4, 1)
+  } else {
+    PICK_NAIVE(3, 0, 4) PICK_NAIVE(3, 2, 4) PICK_NAIVE(2, 0, 4) PICK_NAIVE(2, 2, 4)
+  }
+#undef PICK_NAIVE
   if (F == TECS_FINDER_DELAUNAY && !sym) {
     if (D == 3 && FO == 0) return k_pass<3, 5, 0>;
     if (D == 3 && FO == 1) return k_pass<3, 5, 1>;
@@ -501,7 +523,10 @@ int enqueue_pass(tecs_sim* s, PassArgs a, int& K) {
   if (!fn) return fail("unsupported finder/force/dims combination");
   if (s->d.finder >= TECS_FINDER_NAIVE_DELAUNAY && enqueue_delaunay_mult(s, a, K)) return -1;
   PROF_BEGIN(s);
-  fn<<<ceil_div(L ? L : 1, kPassThreads), kPassThreads, 0, s->stream>>>(s->g, s->fp, a);
+  if (!sym && !s->binned && s->d.finder != TECS_FINDER_DELAUNAY)
+    fn<<<ceil_div(L ? L : 1, kNaiveThreads / 32 * naive_cells(s)), kNaiveThreads, 0, s->stream>>>(s->g, s->fp, a);
+  else
+    fn<<<ceil_div(L ? L : 1, kPassThreads), kPassThreads, 0, s->stream>>>(s->g, s->fp, a);
   PROF_END(s, a.mode == kStore ? "k_pass_store" : a.mode == kEulerFused ? "k_pass_euler"
               : a.mode == kHeun1Fused ? "k_pass_heun1" : "k_pass_heun2");
   K += 1;
