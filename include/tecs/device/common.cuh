@@ -24,16 +24,31 @@ struct GridP {
   int ext[3];       // ceil((max - min) / bin_size), 1 for unused dimensions
   int R;            // search radius in bins, ceil(cutoff * inv_bin)
   unsigned nbins;   // product of extents
+  uint2 div_x, div_y;  // division of a bin number by ext[0], ext[1] (grid_div)
   int pow2;         // bin_size is a power of two: (p - min) / bin_size == (p - min) * inv_bin exactly
 };
 
-// Sets g.pow2 from g.bin_size (host side, after bin_size and inv_bin are set).
+// Division of n < 2^31 by an invariant d as a multiplication and a shift
+// (Granlund and Montgomery, "Division by Invariant Integers using
+// Multiplication", 1994): with s = ceil(log2 d) and m = ceil(2^(31 + s) / d),
+// floor(n / d) = (n m) >> (31 + s).
+inline uint2 grid_divisor(unsigned d) {
+  unsigned s = 0;
+  while ((1ull << s) < d) ++s;
+  return make_uint2((unsigned)(((1ull << (31 + s)) + d - 1) / d), s);
+}
+__device__ __forceinline__ unsigned grid_div(unsigned n, uint2 d) { return __umulhi(n << 1, d.x) >> d.y; }
+
+// Sets g.pow2 from g.bin_size and the divisors from the extents (host side,
+// after those are set).
 // Dividing by 2^k and multiplying by 2^-k round the same real number, so the
 // two forms of the bin coordinate agree bit for bit.
-inline void grid_set_pow2(GridP& g) {
+inline void grid_set_constants(GridP& g) {
   int e = 0;
   const float m = std::frexp(g.bin_size, &e);
   g.pow2 = (m == 0.5f && g.inv_bin * g.bin_size == 1.0f) ? 1 : 0;
+  g.div_x = grid_divisor((unsigned)g.ext[0]);
+  g.div_y = grid_divisor((unsigned)g.ext[1]);
 }
 
 // Built-in force descriptor plus the pair predicates' constants.
@@ -71,6 +86,24 @@ __device__ __forceinline__ unsigned flatten(const GridP& g, const int* c) {
   if (D >= 2) b += (unsigned)c[1] * (unsigned)g.ext[0];
   if (D >= 3) b += (unsigned)c[2] * ((unsigned)g.ext[0] * (unsigned)g.ext[1]);
   return b;
+}
+
+// Two floats in one 64-bit register (the low one first); the packed
+// operations round each half as the scalar ones do.
+__device__ __forceinline__ unsigned long long f32x2_pack(float lo, float hi) {
+  return (unsigned long long)__float_as_uint(lo) | ((unsigned long long)__float_as_uint(hi) << 32);
+}
+__device__ __forceinline__ float f32x2_lo(unsigned long long v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float f32x2_hi(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ unsigned long long f32x2_sub(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f32x2_mul(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
 __device__ __forceinline__ unsigned id_of(const float4& v) { return __float_as_uint(v.w); }

@@ -71,8 +71,6 @@ struct PassArgs {
   // pair capture hook
   uint2* pairs;
   unsigned long long pair_cap;
-  // Gabriel fast path allowed (gabriel_coefficient <= 0.9 and bin size >= cutoff)
-  int gabriel_fast;
   // cell ids of the sorted slots (binned finders keep the bin key in X.w);
   // null when X.w holds the id (naive finders)
   const unsigned* Bid;
@@ -1068,122 +1066,22 @@ __device__ __forceinline__ void pass_epilogue(const GridP& g, const PassArgs& a,
 // A witness k that blocks the pair (i, j) lies inside the ball of radius
 // r = c*d/2 around the midpoint m, and |x_i - m| = d/2, so |x_k - x_i| < d(1+c)/2.
 // For c <= 0.9 and d < cutoff that is < 0.95 * cutoff: every witness is itself
-// one of i's in-cutoff neighbours, found in i's 27 candidate bins.  The pass
-// therefore collects i's in-cutoff neighbours (candidate order = the
-// reference's summation order) into shared memory and tests each pair against
-// the others, keeping the reference's bin-range restriction on k exactly
-// (binned_gabriel.hpp:142-207).  If a cell has more than kMaxNb neighbours, or
-// a ball's bin range leaves i's 3x3x3 block, the cell takes the general path.
-constexpr int kMaxNb = 16;
+// one of i's in-cutoff neighbours, found in i's 27 candidate bins.  The
+// cooperative pass (k_pass_gabriel) therefore lists i's in-cutoff neighbours
+// (candidate order = the reference's summation order) in shared memory and
+// tests each pair against the others, keeping the reference's bin-range
+// restriction on k exactly (binned_gabriel.hpp:142-207).  A cell with more
+// than kMaxNb neighbours takes the general path.
+constexpr int kMaxNb = 24;     // (4 on average at one cell per bin, 12 in packed tissue; a count is a class: at most 31)
+constexpr int kPool = 224;     // neighbours of a warp's cells at a time (about 130 at one cell per bin)
 // Threads (cells) per block of the cooperative passes: three warps.  The
-// block's shared memory (about 30 KB) then lets seven blocks share an SM, 672
+// block's shared memory (about 24 KB) then lets nine blocks share an SM, 864
 // cells, so that a 100k-cell pass runs in a single wave on 152 SMs.
 constexpr int kPassThreads = 96;
 // Position arrays that the cooperative pass scans hold this many float4 past
-// their capacity: the candidate scan reads whole rounds past a row's end (at
-// most 31 slots) and masks the extra slots off.
+// their capacity: the candidate scan reads rounds of four places past a
+// list's end and leaves their bits out.
 constexpr unsigned kRowPad = 64;
-
-// nb: room for MAXN neighbours at a stride of STRIDE (the block size)
-template <int D, int FORCE, int MAXN = kMaxNb, int STRIDE = kPassThreads>
-__device__ __forceinline__ bool gabriel_cell_fast(const GridP& g, const ForceP& fp, const PassArgs& a, unsigned i,
-                                                  const float* xi, float2 pi, unsigned idi, Acc& acc,
-                                                  float4* nb) {
-  int bc[3] = {0, 0, 0};
-  bin_coords_div<D>(g, xi, bc);
-  int cnt = 0;
-  const int z0 = D >= 3 ? -1 : 0, z1 = D >= 3 ? 1 : 0;
-  for (int dz = z0; dz <= z1; ++dz) {
-    const int cz = D >= 3 ? bc[2] + dz : 0;
-    if (D >= 3 && (cz < 0 || cz >= g.ext[2])) continue;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int cy = bc[1] + dy;
-      if (cy < 0 || cy >= g.ext[1]) continue;
-      const int x0 = max(bc[0] - 1, 0), x1 = min(bc[0] + 1, g.ext[0] - 1);
-      int c0[3] = {x0, cy, cz};
-      const unsigned b0 = flatten<D>(g, c0);
-      // boundaries of the (up to) three bins of this row
-      const unsigned o0 = __ldg(&a.off[b0]);
-      const unsigned o1 = __ldg(&a.off[b0 + 1]);
-      const unsigned o2 = x1 >= x0 + 1 ? __ldg(&a.off[b0 + 2]) : o1;
-      const unsigned o3 = x1 >= x0 + 2 ? __ldg(&a.off[b0 + 3]) : o2;
-      for (unsigned j = o0; j < o3; ++j) {
-        if (j == i) continue;
-        const float4 vj = __ldg(&a.X[j]);
-        const float e0 = xi[0] - vj.x, e1 = xi[1] - vj.y;
-        float d2 = e0 * e0 + e1 * e1;
-        if (D >= 3) { const float e2 = xi[2] - vj.z; d2 = d2 + e2 * e2; }
-        if (d2 >= fp.rc2) continue;
-        if (cnt == MAXN) return false;
-        const int rx = x0 + (j >= o1 ? 1 : 0) + (j >= o2 ? 1 : 0) - bc[0];
-        const unsigned code = (unsigned)(rx + 1) | ((unsigned)(dy + 1) << 2) | ((unsigned)(dz + 1) << 4);
-        nb[cnt * STRIDE] = make_float4(vj.x, vj.y, vj.z, __uint_as_float((j << 6) | code));
-        ++cnt;
-      }
-    }
-  }
-  // pass over the pairs: Gabriel test against the other neighbours
-  unsigned accepted = 0u;
-  for (int q = 0; q < cnt; ++q) {
-    const float4 vj = nb[q * STRIDE];
-    float disp[3];
-    disp[0] = xi[0] - vj.x;
-    disp[1] = xi[1] - vj.y;
-    disp[2] = D >= 3 ? xi[2] - vj.z : 0.f;
-    float d2 = disp[0] * disp[0] + disp[1] * disp[1];
-    if (D >= 3) d2 = d2 + disp[2] * disp[2];
-    // midpoint ball and its bin range, relative to i's bin
-    float m[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-    for (int d = 0; d < D; ++d) m[d] = xi[d] - disp[d] * 0.5f;
-    const float rsq = d2 * fp.gab_factor;
-    const float r = sqrtf(rsq);
-    int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      lo[d] = clampi((int)floorf((m[d] - r - g.mn[d]) * g.inv_bin), g.ext[d] - 1) - bc[d];
-      hi[d] = clampi((int)floorf((m[d] + r - g.mn[d]) * g.inv_bin), g.ext[d] - 1) - bc[d];
-      if (lo[d] < -1 || hi[d] > 1) return false;
-    }
-    bool blocked = false;
-    for (int w = 0; w < cnt && !blocked; ++w) {
-      if (w == q) continue;
-      const float4 vk = nb[w * STRIDE];
-      const unsigned code = __float_as_uint(vk.w) & 63u;
-      const int rx = (int)(code & 3u) - 1, ry = (int)((code >> 2) & 3u) - 1, rz = (int)((code >> 4) & 3u) - 1;
-      if (rx < lo[0] || rx > hi[0] || ry < lo[1] || ry > hi[1]) continue;
-      if (D >= 3 && (rz < lo[2] || rz > hi[2])) continue;
-      const float f0 = vk.x - m[0], f1 = vk.y - m[1];
-      float s = f0 * f0 + f1 * f1;
-      if (D >= 3) { const float f2 = vk.z - m[2]; s = s + f2 * f2; }
-      if (s < rsq) blocked = true;
-    }
-    if (!blocked) accepted |= 1u << q;
-  }
-  // forces of the accepted pairs, in candidate (= reference summation) order
-  Acc loc = {{0.f, 0.f, 0.f}, {0.f, 0.f}};
-  while (accepted) {
-    const int q = __ffs(accepted) - 1;
-    accepted &= accepted - 1u;
-    const float4 vj = nb[q * STRIDE];
-    const unsigned j = __float_as_uint(vj.w) >> 6;
-    float disp[3];
-    disp[0] = xi[0] - vj.x;
-    disp[1] = xi[1] - vj.y;
-    disp[2] = D >= 3 ? xi[2] - vj.z : 0.f;
-    float d2 = disp[0] * disp[0] + disp[1] * disp[1];
-    if (D >= 3) d2 = d2 + disp[2] * disp[2];
-    if (a.pairs) {
-      unsigned long long s = atomicAdd(&a.ctr->pair_count, 1ull);
-      if (s < a.pair_cap) a.pairs[s] = make_uint2(idi, id_at(a.X, a.Bid, j));
-    }
-    const float dist = sqrtf(d2);
-    const float2 pj = (FORCE == 2 && a.P) ? __ldg(&a.P[j]) : make_float2(0.f, 0.f);
-    pair_force<D, FORCE>(fp, disp, dist, pi, pj, loc);
-  }
-  acc = loc;
-  return true;
-}
 
 template <int D, int FINDER, int FORCE>
 __device__ __forceinline__ void cell_general(const GridP& g, const ForceP& fp, const PassArgs& a, unsigned n, unsigned i,
@@ -1203,15 +1101,7 @@ static __global__ void __launch_bounds__(kPassThreads) k_pass(GridP g, ForceP fp
     xi[0] = vi.x; xi[1] = vi.y; xi[2] = vi.z;
     if (a.P) pi = a.P[i];
     const unsigned idi = id_at(a.X, a.Bid, i);
-    if (FINDER == 3 && a.gabriel_fast) {
-      __shared__ float4 nbuf[kMaxNb * kPassThreads];
-      if (!gabriel_cell_fast<D, FORCE>(g, fp, a, i, xi, pi, idi, acc, &nbuf[threadIdx.x])) {
-        // nothing was recorded or accumulated yet: redo the cell the general way
-        cell_general<D, FINDER, FORCE>(g, fp, a, n, i, xi, pi, idi, acc);
-      }
-    } else {
-      cell_general<D, FINDER, FORCE>(g, fp, a, n, i, xi, pi, idi, acc);
-    }
+    cell_general<D, FINDER, FORCE>(g, fp, a, n, i, xi, pi, idi, acc);
   }
   pass_epilogue<D>(g, a, active, n, i, xi, vi, pi, acc);
 }
@@ -1591,32 +1481,84 @@ int prepare_user_pass(int device) {
 }
 
 // ---------------------------------------------------------------------------
-// Warp-cooperative Gabriel pass (spring laws and the 3-D polarity law).
-//
-// Same pair semantics as gabriel_cell_fast, reorganised so that the lanes stay
-// busy: (1) each thread collects its cell's in-cutoff neighbours into shared
-// memory, in candidate order; (2) each warp lists every (cell, neighbour)
-// pair of its 32 cells -- sorted by the cell's neighbour count, so the
-// Gabriel loops of a round of pairs run the same length -- and its lanes take
-// pairs round-robin for the Gabriel test, setting accept bits per cell; (3)
-// the same for the pair forces, each written over its candidate slot; (4) each thread
-// adds its cell's accepted contributions in candidate order -- the
-// reference's summation order, so the sums stay bit-identical.  Cells with
-// more neighbours than the slots, or whose witness ball leaves the 3x3x3 bin
-// block, take the general path in phase 4.
-// Candidate slot (q, cell c) in shared memory, XOR-swizzled so that threads
-// reading different q of the same cell hit different banks.
-__device__ __forceinline__ int cix(int q, int c) { return q * kPassThreads + (c ^ q); }
-
+// Warp-cooperative pass of the binned finders (spring laws and the 3-D
+// polarity law): same pair semantics as cell_general on the fast path's
+// geometry, reorganised so that the lanes stay busy.  Its phases and the
+// reasons for them stand in pass_gabriel_body.inc.
 // FINDER 3: binned Gabriel; FINDER 1: binned all-pairs (i's bin by
 // multiplication, binned_all_pairs.hpp:103-109, and every in-cutoff pair
-// accepted: no phase 2).
+// accepted: no witness test).
+
+// binned_gabriel.hpp:142-153: a witness in the ball (m, r) blocks only from a
+// bin of the ball's bin range.
+template <int D>
+struct BallBins {
+  int lo[3], hi[3];
+  __device__ __forceinline__ BallBins(const GridP& g, const float* m, float r) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      lo[d] = clampi((int)floorf((m[d] - r - g.mn[d]) * g.inv_bin), g.ext[d] - 1);
+      hi[d] = clampi((int)floorf((m[d] + r - g.mn[d]) * g.inv_bin), g.ext[d] - 1);
+    }
+  }
+  __device__ __forceinline__ bool holds(const GridP& g, unsigned key) const {
+    const unsigned row = grid_div(key, g.div_x);
+    const int kx = (int)(key - row * (unsigned)g.ext[0]);
+    const int kz = D >= 3 ? (int)grid_div(row, g.div_y) : 0;
+    const int ky = (int)row - kz * g.ext[1];
+    return kx >= lo[0] && kx <= hi[0] && ky >= lo[1] && ky <= hi[1] && (D < 3 || (kz >= lo[2] && kz <= hi[2]));
+  }
+};
+
+#define TECS_WITNESS (FINDER == 3)
+#define TECS_ANY_WITNESS (FINDER == 3)
+#define TECS_PAIR_G(c) g
+#define TECS_PAIR_FP(c) fp
+#define TECS_PAIR_KEY0(c) 0u
+#define TECS_SPRING(fpc) (FORCE != 0)
+#define TECS_POLAR(fpc) true
+#define TECS_CAPTURING (a.pairs != nullptr)
+#define TECS_CAPTURE(c, jj)                                                                   \
+  if (a.pairs) {                                                                              \
+    const unsigned long long s_ = atomicAdd(&a.ctr->pair_count, 1ull);                        \
+    if (s_ < a.pair_cap)                                                                      \
+      a.pairs[s_] = make_uint2(id_at(a.X, a.Bid, i - (unsigned)lane + (c)), id_at(a.X, a.Bid, (jj))); \
+  }
+#define TECS_PASS_BODY(BLK)                                                                   \
+  static_assert(FORCE <= 1 || (FORCE == 2 && D == 3), "spring laws, or the 3-D polarity law"); \
+  static_assert(FINDER == 1 || FINDER == 3, "the binned finders");                            \
+  constexpr bool POL = FORCE == 2;                                                            \
+  constexpr int TB = kPassThreads;                                                            \
+  const unsigned n = a.ctr->n;                                                                \
+  const unsigned i = (BLK)*TB + threadIdx.x;                                                  \
+  const bool run = i < n;                                                                     \
+  const float4* const X = a.X;                                                                \
+  const float2* const P = a.P;                                                                \
+  const unsigned* const off = a.off;                                                          \
+  const float rc2 = fp.rc2;                                                                   \
+  float xi[3] = {0.f, 0.f, 0.f};                                                              \
+  float4 vi = make_float4(0.f, 0.f, 0.f, 0.f);                                                \
+  float2 pi = make_float2(0.f, 0.f);                                                          \
+  int bc[3] = {0, 0, 0};                                                                      \
+  bool fb = false;                                                                            \
+  Acc acc = {{0.f, 0.f, 0.f}, {0.f, 0.f}};                                                    \
+  if (run) {                                                                                  \
+    vi = __ldg(&X[i]);                                                                        \
+    xi[0] = vi.x; xi[1] = vi.y; xi[2] = vi.z;                                                 \
+    if (P) pi = P[i];                                                                         \
+    if (FINDER == 1) bin_coords_mul<D>(g, xi, bc);                                            \
+    else bin_coords_div<D>(g, xi, bc);                                                        \
+  }
+#define TECS_PASS_END                                                                         \
+  if (fb) cell_general<D, FINDER, FORCE>(g, fp, a, n, i, xi, pi, id_at(a.X, a.Bid, i), acc);  \
+  pass_epilogue<D>(g, a, run, n, i, xi, vi, pi, acc);
+
 // The grid pass: block blockIdx.x's cells.
 template <int D, int FORCE, int FINDER = 3>
-static __global__ void __launch_bounds__(kPassThreads) k_pass_gabriel(GridP g, ForceP fp, PassArgs a) {
-#define TECS_PASS_BLOCK blockIdx.x
+static __global__ void __launch_bounds__(kPassThreads, FORCE == 2 ? 6 : 9) k_pass_gabriel(GridP g, ForceP fp, PassArgs a) {
+  TECS_PASS_BODY(blockIdx.x)
 #include "pass_gabriel_body.inc"
-#undef TECS_PASS_BLOCK
+  TECS_PASS_END
 }
 
 // One block's cells blk * kPassThreads .. (only warp-level synchronisation,
@@ -1624,10 +1566,21 @@ static __global__ void __launch_bounds__(kPassThreads) k_pass_gabriel(GridP g, F
 template <int D, int FORCE, int FINDER = 3>
 __device__ __forceinline__ void pass_gabriel_block(const GridP& g, const ForceP& fp, const PassArgs& a,
                                                    const unsigned blk) {
-#define TECS_PASS_BLOCK blk
+  TECS_PASS_BODY(blk)
 #include "pass_gabriel_body.inc"
-#undef TECS_PASS_BLOCK
+  TECS_PASS_END
 }
+#undef TECS_WITNESS
+#undef TECS_ANY_WITNESS
+#undef TECS_PAIR_G
+#undef TECS_PAIR_FP
+#undef TECS_PAIR_KEY0
+#undef TECS_SPRING
+#undef TECS_POLAR
+#undef TECS_CAPTURING
+#undef TECS_CAPTURE
+#undef TECS_PASS_BODY
+#undef TECS_PASS_END
 
 // Symmetric finders (…_symmetric.hpp): only j with a smaller id, +delta to the
 // evaluating cell and -delta to j for every field.  Float atomics: the

@@ -141,299 +141,74 @@ static __global__ void k_eorder_gather(const unsigned* __restrict__ off, unsigne
 }
 
 // ---------------------------------------------------------------------------
-// the force pass over all slots: k_pass_gabriel's per-warp phases with each
-// cell's simulation parameters taken from the table
+// the force pass over all slots: the phases of k_pass_gabriel
+// (pass_gabriel_body.inc) with each cell's simulation parameters taken from
+// the table -- cells of different simulations share a warp at region borders
 
-// POL: some resident simulation carries polarity; their cells then take the
-// cooperative path with the polarity law, its pair terms added in the ordered
-// sums -- spring-only engines use the instance without that branch.
+// POL: some resident simulation carries polarity; spring-only engines use the
+// instance without the polarity law's terms.
 // TB: threads per block (64, 96 or 128; the autotuner's choice).
-template <int TB>
-__device__ __forceinline__ int ecix(int q, int c) { return q * TB + (c ^ q); }
+#define TECS_WITNESS gab
+#define TECS_ANY_WITNESS true
+#define TECS_PAIR_G(c) e.table[hsim[warp * 32 + (c)]].g
+#define TECS_PAIR_FP(c) e.table[hsim[warp * 32 + (c)]].fp
+#define TECS_PAIR_KEY0(c) e.table[hsim[warp * 32 + (c)]].bin_base
+#define TECS_SPRING(fpc) ((fpc).force != TECS_FORCE_NONE)
+#define TECS_POLAR(fpc) ((fpc).force == TECS_FORCE_POLARITY)
+#define TECS_CAPTURING false
+#define TECS_CAPTURE(c, jj)
 
 template <int PASS, bool POL, int TB>
-static __global__ void __launch_bounds__(TB) k_epass(EngArgs e) {
-  constexpr int NB = kMaxNb;  // neighbour slots per cell (more: the per-thread path)
-  __shared__ float4 cand[NB * TB];
-  __shared__ float4 home[TB];
-  __shared__ unsigned short pinfo[NB * TB];
-  __shared__ unsigned short wcls[TB / 32][NB + 1];  // pairs per (warp, neighbour count)
-  __shared__ unsigned amask[TB];
-  __shared__ unsigned char ncnt[TB];
+static __global__ void __launch_bounds__(TB, (POL ? 576 : 864) / TB) k_epass(EngArgs e) {
+  constexpr int D = 3;
   __shared__ unsigned hsim[TB];
   const unsigned n = e.off[e.nb_total];
-  const int t = threadIdx.x;
-  const unsigned i = blockIdx.x * TB + t;
+  const unsigned i = blockIdx.x * TB + threadIdx.x;
   const bool active = i < n;
   const unsigned sim = active ? e.Bsim[i] : 0u;
+  hsim[threadIdx.x] = sim;
   const SimSlot& sl = e.table[sim];
+  const GridP& g = sl.g;
+  const float4* const X = e.X;
+  const float2* const P = e.P;
+  const unsigned* const off = e.off + sl.bin_base;  // the slot's own bins, indexed by its local flat index
+  const float rc2 = sl.fp.rc2;
   // Euler simulations take one pass; their second-pass cells sit out
   const bool run = active && (PASS == 1 || sl.integrator == TECS_HEUN);
-  const bool polar = run && sl.has_pol;
   const bool gab = sl.finder == TECS_FINDER_BINNED_GABRIEL;
   float xi[3] = {0.f, 0.f, 0.f};
   float4 vi = make_float4(0.f, 0.f, 0.f, 0.f);
   float2 pi = make_float2(0.f, 0.f);
   int bc[3] = {0, 0, 0};
-  int cnt = 0;
-  bool fb = (polar && !POL) || (run && gab && !sl.gabriel_fast);
+  bool fb = (run && sl.has_pol && !POL) || (run && gab && !sl.gabriel_fast);
+  Acc acc = {{0.f, 0.f, 0.f}, {0.f, 0.f}};
   if (run) {
-    vi = __ldg(&e.X[i]);
+    vi = __ldg(&X[i]);
     xi[0] = vi.x; xi[1] = vi.y; xi[2] = vi.z;
-    if (sl.has_pol) pi = e.P[i];
+    if (sl.has_pol) pi = P[i];
     // i's own bin: division for the Gabriel finder (grid.hpp:222-230),
     // multiplication for BinnedAllPairs (binned_all_pairs.hpp:103-109)
-    if (gab) bin_coords_div<3>(sl.g, xi, bc);
-    else bin_coords_mul<3>(sl.g, xi, bc);
+    if (gab) bin_coords_div<3>(g, xi, bc);
+    else bin_coords_mul<3>(g, xi, bc);
   }
-  if (run && !fb) {
-    const GridP& g = sl.g;
-    const int x0 = max(bc[0] - 1, 0), x1 = min(bc[0] + 1, g.ext[0] - 1);
-    unsigned rlo[9], rhi[9], rb0[9];
-#pragma unroll
-    for (int r = 0; r < 9; ++r) {
-      const int cy = bc[1] + r % 3 - 1, cz = bc[2] + r / 3 - 1;
-      const bool ok = cy >= 0 && cy < g.ext[1] && cz >= 0 && cz < g.ext[2];
-      int c0[3] = {x0, ok ? cy : 0, ok ? cz : 0};
-      const unsigned b0 = sl.bin_base + flatten<3>(g, c0);
-      rb0[r] = b0;
-      rlo[r] = ok ? __ldg(&e.off[b0]) : 0u;
-      rhi[r] = ok ? __ldg(&e.off[b0 + (unsigned)(x1 - x0) + 1u]) : 0u;
-    }
-    const int rxo = x0 - bc[0] + 1;
-    const float rc2 = sl.fp.rc2;
-    // as k_pass_gabriel: the three rows of each z-plane scanned together, two
-    // candidates at a time, in-cutoff ones appended in candidate order
-#pragma unroll
-    for (int g0 = 0; g0 < 9; g0 += 3) {
-      unsigned len[3];
-      unsigned lmax = 0u;
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        len[q] = rhi[g0 + q] - rlo[g0 + q];
-        lmax = max(lmax, len[q]);
-      }
-      if (lmax > 32u) fb = true;
-      if (fb) continue;
-      unsigned m[3] = {0u, 0u, 0u};
-      for (unsigned o = 0; o < lmax; o += 2u) {
-        float4 v[3][2];
-#pragma unroll
-        for (int q = 0; q < 3; ++q)
-#pragma unroll
-          for (int k = 0; k < 2; ++k)
-            v[q][k] = __ldg(&e.X[len[q] ? rlo[g0 + q] + min(o + k, len[q] - 1u) : i]);
-#pragma unroll
-        for (int q = 0; q < 3; ++q)
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const unsigned j = rlo[g0 + q] + o + k;
-            const float e0 = xi[0] - v[q][k].x, e1 = xi[1] - v[q][k].y, e2 = xi[2] - v[q][k].z;
-            float d2 = e0 * e0 + e1 * e1;
-            d2 = d2 + e2 * e2;
-            if (o + k < len[q] && j != i && d2 < rc2) m[q] |= 1u << (o + k);
-          }
-      }
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const int r = g0 + q;
-        const unsigned rowcode = 3u * (unsigned)(r % 3) + 9u * (unsigned)(r / 3);
-        unsigned mm = m[q];
-        if (cnt + __popc(mm) > NB) { fb = true; break; }
-        while (mm) {
-          const unsigned j = rlo[r] + (unsigned)(__ffs(mm) - 1);
-          mm &= mm - 1u;
-          const float4 v = __ldg(&e.X[j]);
-          const unsigned rx = (unsigned)((int)(__float_as_uint(v.w) - rb0[r]) + rxo);
-          cand[ecix<TB>(cnt, t)] = make_float4(v.x, v.y, v.z, __uint_as_float((j << 5) | (rowcode + rx)));
-          ++cnt;
-        }
-      }
-    }
-  }
-  if (fb) cnt = 0;
-  home[t] = make_float4(xi[0], xi[1], xi[2],
-                        __uint_as_float((unsigned)bc[0] | ((unsigned)bc[1] << 10) | ((unsigned)bc[2] << 20)));
-  hsim[t] = sim;
-  ncnt[t] = (unsigned char)cnt;
-  // Phases 2-4 run per warp over the warp's own 32 cells, as in
-  // k_pass_gabriel.  Only cells of Gabriel slots with two or more neighbours
-  // need the Gabriel test (a single neighbour has no witness; all-pairs
-  // slots accept every in-cutoff pair); their pairs are listed sorted by the
-  // cell's neighbour count, so that the witness loops of a round run the
-  // same length.
-  const int lane = t & 31, warp = t >> 5;
-  unsigned short* const wp = pinfo + warp * 32 * NB;
-  const bool tested = run && !fb && gab && cnt >= 2;
-  const int tcnt = tested ? cnt : 0;
-  int P = 0;
-  {
-    if (lane <= NB) wcls[warp][lane] = 0;
-    __syncwarp();
-    const unsigned same = __match_any_sync(0xffffffffu, tcnt);
-    const int rank = __popc(same & ((1u << lane) - 1u));
-    if (rank == 0) wcls[warp][tcnt] = (unsigned short)(__popc(same) * (unsigned)tcnt);
-    amask[t] = tested ? 0u : (1u << cnt) - 1u;  // cnt <= 16; 0 for fallback and idle cells
-    __syncwarp();
-    const unsigned tot = lane <= NB ? (unsigned)wcls[warp][lane] : 0u;
-    unsigned incl = tot;
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    P = (int)__shfl_sync(0xffffffffu, incl, NB);
-    const int base = (int)__shfl_sync(0xffffffffu, incl - tot, tcnt) + rank * tcnt;
-    for (int q = 0; q < tcnt; ++q) wp[base + q] = (unsigned short)((t << 4) | q);
-  }
-  __syncwarp();
-
-  // ---- Gabriel test, one pair per lane at a time, two witnesses per round
-  for (int p = lane; p < P; p += 32) {
-    const unsigned info = wp[p];
-    const int c = (int)(info >> 4), q = (int)(info & 15u);
-    const SimSlot& cs = e.table[hsim[c]];
-    const float4 h = home[c];
-    const float4 vj = cand[ecix<TB>(q, c)];
-    const float hx[3] = {h.x, h.y, h.z};
-    const float disp[3] = {hx[0] - vj.x, hx[1] - vj.y, hx[2] - vj.z};
-    float d2 = disp[0] * disp[0] + disp[1] * disp[1];
-    d2 = d2 + disp[2] * disp[2];
-    float m[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) m[d] = hx[d] - disp[d] * 0.5f;
-    const float rsq = d2 * cs.fp.gab_factor;
-    const int cc = ncnt[c];
-    unsigned hits = 0u, bit = 1u;
-    for (int w = 0; w < cc; w += 2) {
-      const int w1 = min(w + 1, cc - 1);
-      const float4 vk0 = cand[ecix<TB>(w, c)], vk1 = cand[ecix<TB>(w1, c)];
-      const float f0 = vk0.x - m[0], f1 = vk0.y - m[1], f2 = vk0.z - m[2];
-      const float g0 = vk1.x - m[0], g1 = vk1.y - m[1], g2 = vk1.z - m[2];
-      float sd0 = f0 * f0 + f1 * f1, sd1 = g0 * g0 + g1 * g1;
-      sd0 = sd0 + f2 * f2;
-      sd1 = sd1 + g2 * g2;
-      if (sd0 < rsq) hits |= bit;
-      if (sd1 < rsq) hits |= bit << 1;
-      bit <<= 2;
-    }
-    hits &= ((1u << cc) - 1u) & ~(1u << q);
-    bool blocked = false;
-    if (hits) {
-      // a witness in the ball blocks only from a bin overlapping the ball
-      // (binned_gabriel.hpp:142-153), relative to the cell's bin
-      const unsigned hb = __float_as_uint(h.w);
-      const int hbc[3] = {(int)(hb & 1023u), (int)((hb >> 10) & 1023u), (int)(hb >> 20)};
-      const float r = sqrtf(rsq);
-      int lo[3], hi[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        lo[d] = clampi((int)floorf((m[d] - r - cs.g.mn[d]) * cs.g.inv_bin), cs.g.ext[d] - 1) - hbc[d];
-        hi[d] = clampi((int)floorf((m[d] + r - cs.g.mn[d]) * cs.g.inv_bin), cs.g.ext[d] - 1) - hbc[d];
-      }
-      while (hits && !blocked) {
-        const int w = __ffs(hits) - 1;
-        hits &= hits - 1u;
-        const unsigned code = __float_as_uint(cand[ecix<TB>(w, c)].w) & 31u;
-        const int rel[3] = {(int)(code % 3u) - 1, (int)((code / 3u) % 3u) - 1, (int)(code / 9u) - 1};
-        bool inside = true;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) inside = inside && rel[d] >= lo[d] && rel[d] <= hi[d];
-        blocked = inside;
-      }
-    }
-    if (!blocked) atomicOr(&amask[c], 1u << q);
-  }
-  __syncwarp();
-  // the warp's accepted spring pairs, cell by cell, over the pair list (the
-  // polarity law's pairs are summed term by term in the ordered sums)
-  int PA = 0;
-  {
-    const bool pol_cell = POL && polar && sl.fp.force == TECS_FORCE_POLARITY;
-    const unsigned acc_bits = (fb || pol_cell || !run) ? 0u : amask[t];
-    const int na = __popc(acc_bits);
-    int incl = na;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    PA = __shfl_sync(0xffffffffu, incl, 31);
-    int base = incl - na;
-    __syncwarp();
-    for (unsigned b = acc_bits; b; b &= b - 1u) wp[base++] = (unsigned short)((t << 4) | (__ffs(b) - 1));
-  }
-  __syncwarp();
-  // ---- spring2r forces of the accepted pairs, written over the candidate slot
-  for (int p = lane; p < PA; p += 32) {
-    const unsigned info = wp[p];
-    const int c = (int)((info >> 4) & 127u), q = (int)(info & 15u);
-    const SimSlot& cs = e.table[hsim[c]];
-    const float4 h = home[c];
-    const float4 vj = cand[ecix<TB>(q, c)];
-    const float disp[3] = {h.x - vj.x, h.y - vj.y, h.z - vj.z};
-    float d2 = disp[0] * disp[0] + disp[1] * disp[1];
-    d2 = d2 + disp[2] * disp[2];
-    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float dist = sqrtf(d2);
-    if (cs.fp.force != TECS_FORCE_NONE && dist != 0.0f) {
-      // (displacement * F) / distance; a zero F leaves the sum unchanged
-      const ForceP& fp = cs.fp;
-      const float F = fp.k_rep * fmaxf(fp.r_rep - dist, 0.0f) - fp.k_adh * fmaxf(dist - fp.r_adh, 0.0f);
-      if (F != 0.0f) {
-        f.x = (disp[0] * F) / dist;
-        f.y = (disp[1] * F) / dist;
-        f.z = (disp[2] * F) / dist;
-      }
-    }
-    cand[ecix<TB>(q, c)] = f;
-  }
-  __syncwarp();
-  // ---- ordered per-cell sums
-  Acc acc = {{0.f, 0.f, 0.f}, {0.f, 0.f}};
-  if (run && !fb) {
-    const bool pol_law = POL && polar && sl.fp.force == TECS_FORCE_POLARITY;
-    for (int q = 0; q < cnt; ++q) {
-      if (!((amask[t] >> q) & 1u)) continue;
-      const float4 f = cand[ecix<TB>(q, t)];
-      if (pol_law) {
-        // this pair's spring, bending vector, bending and alignment terms, each
-        // added to the sums in turn (polarity.hpp:131-198 as pair_force adds them)
-        const float disp[3] = {xi[0] - f.x, xi[1] - f.y, xi[2] - f.z};
-        float d2 = disp[0] * disp[0] + disp[1] * disp[1];
-        d2 = d2 + disp[2] * disp[2];
-        const float2 pj = __ldg(&e.P[__float_as_uint(f.w) >> 5]);
-        pair_force<3, 2>(sl.fp, disp, sqrtf(d2), pi, pj, acc);
-        continue;
-      }
-      acc.x[0] = acc.x[0] + f.x;
-      acc.x[1] = acc.x[1] + f.y;
-      acc.x[2] = acc.x[2] + f.z;
-    }
-  }
-  // the warp's sums are read: its candidate columns serve the per-thread
-  // neighbour lists of the overflow path
-  __syncwarp();
+#include "../../include/tecs/device/pass_gabriel_body.inc"
   if (!run) return;
   if (fb) {
     PassArgs pa{};
-    pa.X = e.X;
-    pa.P = sl.has_pol ? e.P : nullptr;
-    pa.off = e.off + sl.bin_base;  // the slot's own bins, indexed by its local flat index
+    pa.X = X;
+    pa.P = sl.has_pol ? P : nullptr;
+    pa.off = off;
     pa.Bid = nullptr;
     const unsigned idi = __ldg(&e.Bid[i]);
     const int force = sl.fp.force;
     if (gab) {
-      if (force == TECS_FORCE_POLARITY) {
-        if (!(sl.gabriel_fast && gabriel_cell_fast<3, 2, NB, TB>(sl.g, sl.fp, pa, i, xi, pi, idi, acc, &cand[t])))
-          cell_general<3, 3, 2>(sl.g, sl.fp, pa, n, i, xi, pi, idi, acc);
-      } else if (force == TECS_FORCE_SPRING2R) {
-        cell_general<3, 3, 1>(sl.g, sl.fp, pa, n, i, xi, pi, idi, acc);
-      } else {
-        cell_general<3, 3, 0>(sl.g, sl.fp, pa, n, i, xi, pi, idi, acc);
-      }
+      if (force == TECS_FORCE_POLARITY) cell_general<3, 3, 2>(g, sl.fp, pa, n, i, xi, pi, idi, acc);
+      else if (force == TECS_FORCE_SPRING2R) cell_general<3, 3, 1>(g, sl.fp, pa, n, i, xi, pi, idi, acc);
+      else cell_general<3, 3, 0>(g, sl.fp, pa, n, i, xi, pi, idi, acc);
     } else {
-      if (force == TECS_FORCE_POLARITY) cell_general<3, 1, 2>(sl.g, sl.fp, pa, n, i, xi, pi, idi, acc);
-      else if (force == TECS_FORCE_SPRING2R) cell_general<3, 1, 1>(sl.g, sl.fp, pa, n, i, xi, pi, idi, acc);
-      else cell_general<3, 1, 0>(sl.g, sl.fp, pa, n, i, xi, pi, idi, acc);
+      if (force == TECS_FORCE_POLARITY) cell_general<3, 1, 2>(g, sl.fp, pa, n, i, xi, pi, idi, acc);
+      else if (force == TECS_FORCE_SPRING2R) cell_general<3, 1, 1>(g, sl.fp, pa, n, i, xi, pi, idi, acc);
+      else cell_general<3, 1, 0>(g, sl.fp, pa, n, i, xi, pi, idi, acc);
     }
   }
   // integrator epilogues (euler.hpp:49-69, heun.hpp:54-98; no COM fix)
@@ -471,6 +246,15 @@ static __global__ void __launch_bounds__(TB) k_epass(EngArgs e) {
   e.PA[i] = pn;
   e.Asim[i] = sim;
 }
+#undef TECS_WITNESS
+#undef TECS_ANY_WITNESS
+#undef TECS_PAIR_G
+#undef TECS_PAIR_FP
+#undef TECS_PAIR_KEY0
+#undef TECS_SPRING
+#undef TECS_POLAR
+#undef TECS_CAPTURING
+#undef TECS_CAPTURE
 
 // Euler cells keep their pass-1 state: nothing to do in pass 2 (handled by `run`).
 
@@ -665,7 +449,8 @@ int tecs_engine_create(const tecs_engine_desc* desc, tecs_engine** out) {
   auto al = [&](void** p, size_t b) { return cudaMalloc(p, b ? b : 16) == cudaSuccess; };
   bool ok = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) == cudaSuccess &&
             cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking) == cudaSuccess;
-  ok = ok && al((void**)&e->A, C * 16) && al((void**)&e->B, C * 16) && al((void**)&e->Xt, C * 16) &&
+  ok = ok && al((void**)&e->A, C * 16) && al((void**)&e->B, (C + kRowPad) * 16) &&
+       al((void**)&e->Xt, (C + kRowPad) * 16) &&
        al((void**)&e->d1, C * 16) && al((void**)&e->PA, C * 8) && al((void**)&e->PB, C * 8) &&
        al((void**)&e->Pt, C * 8) && al((void**)&e->dp1, C * 8) && al((void**)&e->Asim, C * 4) &&
        al((void**)&e->Bsim, C * 4) && al((void**)&e->Bid, C * 4) && al((void**)&e->key, C * 4) &&
@@ -688,6 +473,8 @@ int tecs_engine_create(const tecs_engine_desc* desc, tecs_engine** out) {
          cudaMemsetAsync(e->off, 0, ((size_t)e->NB + 1) * 4, st) == cudaSuccess &&
          cudaMemsetAsync(e->ctr, 0, sizeof(Counters), st) == cudaSuccess &&
          cudaMemsetAsync(e->table, 0, sizeof(SimSlot) * e->S, st) == cudaSuccess &&
+         cudaMemsetAsync(e->B, 0, (C + kRowPad) * 16, st) == cudaSuccess &&
+         cudaMemsetAsync(e->Xt, 0, (C + kRowPad) * 16, st) == cudaSuccess &&
          cudaMemsetAsync(e->PA, 0, C * 8, st) == cudaSuccess && cudaMemsetAsync(e->PB, 0, C * 8, st) == cudaSuccess &&
          cudaStreamSynchronize(st) == cudaSuccess;
   }
@@ -781,7 +568,7 @@ int tecs_engine_add(tecs_engine* e, const tecs_sim_desc* d, const float* positio
   }
   if (g.R != 1 || g.bin_size < d->cutoff) return fail("the engine needs bin_size_scale >= 1");
   g.nbins = (unsigned)nb;
-  grid_set_pow2(g);
+  grid_set_constants(g);
   unsigned base = 0;
   if (bins_alloc(e, g.nbins, &base)) return fail("engine bin capacity exhausted");
   ForceP& f = sl.fp;

@@ -147,7 +147,7 @@ int tecs_grid_create(int dims, const float* min_bounds, const float* max_bounds,
   }
   if (nb > (1ull << 31)) { delete G; return set_last_error("bin grid too large"); }
   g.nbins = (unsigned)nb;
-  grid_set_pow2(g);
+  grid_set_constants(g);
   const size_t cap = G->cap, len = (size_t)g.nbins + 1;
   auto al = [](void** p, size_t b) { return cudaMalloc(p, b ? b : 16) == cudaSuccess; };
   bool ok = cudaStreamCreateWithFlags(&G->stream, cudaStreamNonBlocking) == cudaSuccess;

@@ -271,12 +271,9 @@ int prof_mark(tecs_sim* s, int which, const char* name) {
   if (prof_mark((s), 1, (name))) return -1
 
 
-// The cooperative Gabriel pass needs the fast-path geometry and packs bin
-// coordinates in 10 bits and slots in 27 bits.
-bool coop_geometry(const tecs_sim* s) {
-  return s->g.R == 1 && s->g.bin_size >= s->d.cutoff && s->g.ext[0] <= 1024 && s->g.ext[1] <= 1024 &&
-         s->g.ext[2] <= 1024 && s->d.capacity < (1u << 27);
-}
+// The cooperative pass needs the fast-path geometry: the candidates of a cell
+// in the 3^dims bins around its own.
+bool coop_geometry(const tecs_sim* s) { return s->g.R == 1 && s->g.bin_size >= s->d.cutoff; }
 // The built-in binned pass over the grid is the cooperative one
 // (k_pass_gabriel): all-pairs on its geometry, Gabriel also with c <= 0.9.
 bool coop_pass(const tecs_sim* s) {
@@ -369,8 +366,6 @@ PassArgs base_args(const tecs_sim* s, float dt, double dt64 = 0.0) {
   a.div_slot = s->div_slot;
   a.A = s->A;
   a.PA = s->d.has_polarity ? s->PA : nullptr;
-  // the fast Gabriel path needs every witness inside i's cutoff ball and 3x3x3 bin block
-  a.gabriel_fast = (s->d.gabriel_coefficient <= 0.9f && s->g.R == 1 && s->g.bin_size >= s->d.cutoff) ? 1 : 0;
   a.count_next = s->fuse_count ? 1 : 0;
   a.Bid = s->binned ? s->Bid : nullptr;
   a.key = s->key;
@@ -856,7 +851,7 @@ int tecs_sim_create(const tecs_sim_desc* desc, tecs_sim** out) {
   if (binned_finder && nb > (1ull << 31)) { delete s; return fail("bin grid too large"); }
   if (!binned_finder && nb > (1ull << 31)) nb = 1ull << 31;
   g.nbins = (unsigned)nb;
-  grid_set_pow2(g);
+  grid_set_constants(g);
   ForceP& f = s->fp;
   f.force = desc->force;
   f.k_rep = desc->k_rep; f.r_rep = desc->r_rep; f.k_adh = desc->k_adh; f.r_adh = desc->r_adh; f.k_pol = desc->k_pol;
@@ -1614,7 +1609,7 @@ extern "C" int tecs_force_pass_noalloc(const tecs_sim_desc* desc, const float* d
     return fail("tecs_force_pass_noalloc: " + std::to_string(nb) + " bins exceed the allocation-free limit of " +
                 std::to_string(kNoallocMaxBins));
   g.nbins = (unsigned)nb;
-  grid_set_pow2(g);
+  grid_set_constants(g);
   ForceP& f = s.fp;
   f.force = desc->force;
   f.k_rep = desc->k_rep; f.r_rep = desc->r_rep; f.k_adh = desc->k_adh; f.r_adh = desc->r_adh; f.k_pol = 0.f;
