@@ -1,0 +1,549 @@
+// delaunay_local.cuh -- the Delaunay finder's fast path: cells whose star lies
+// within a gathered neighbourhood, one warp per cell, without FP64 searches.
+//
+// delaunay_star.cuh walks a cell's Voronoi cell in double, one search of the
+// grid after the other; FP64 is scarce on this part (about two lanes an SM and
+// clock) and the searches depend on each other.  Here a warp gathers the
+// points of a box of bins around the cell once (relative to it, in shared
+// memory), finds the cell's partners from them in float with all lanes, and
+// keeps the result only where it is certain; any doubt -- a point nearer to a
+// circle or sphere than the rounding, a sphere that reaches out of the gathered
+// ball, a hull face, a duplicate -- hands the cell on: to a second search (2-D:
+// over a larger box; 3-D: that looks up what lies beyond the ball), then to the
+// walk in double.
+//
+// 3-D.  For an in-cutoff j the Voronoi face of (i, j) is a polygon in their
+// bisector plane.  Each third point k bounds it by a line; a lane takes a k
+// and cuts its line by every other point, which leaves an interval if (i, j,
+// k) is a triangle of the triangulation, with the fourth points of its two
+// tetrahedra at the ends.  Each tetrahedron is met from both of its third
+// points (checked), so the tetrahedra around (i, j) form a closed ring, and
+// each one's circumcentre is solved in double and every gathered point tested
+// against its sphere with a margin above the float rounding: empty spheres are
+// the Delaunay tetrahedra, whichever way they were found.
+//
+// 2-D.  The reference's float test decides (delaunay_star.cuh, 3): every
+// triangle (i, j, k) of an in-cutoff j and a gathered k is put to it, the lanes
+// taking the k.  The cell's own triangles are found in float as well (each
+// lane takes a neighbour and the nearest parameter on either side), to make
+// sure that the circles, with the tolerance inside which delaunay_star.cuh looks for
+// further third points, lie within the gathered disk.
+//
+// What bounds it: instruction issue, then the latency of the few cells left to
+// the walk.  40k cells in space, one pass: 54 ms (the walk for every cell) ->
+// 3.3 (1.4 the first search, 0.9 the second over 7 % of the cells, 0.8 the
+// walk of 9 cells); 30k in the plane, two passes: 32 -> 3.7 ms.
+#pragma once
+
+#include "delaunay_star.cuh"
+
+namespace tecs {
+namespace dl {
+
+constexpr int kLocalThreads = 128;
+constexpr unsigned kNoEnd = 0xffffu;
+// A point's power (|v|^2 - 2 x.v) / 2 in a sphere about x through the cell has
+// to exceed kPowerV |v|^2 / 2 + kPowerX |x|^2.  Its float error (u = 6e-8 for
+// each product and sum, for v and for x) is at most 6 u (|x| |v| + |v|^2 / 2)
+// <= 1.8e-7 |x|^2 + 3.6e-7 |v|^2: the margin is five times that.
+constexpr float kPowerV = 4.0e-6f, kPowerX = 1.0e-6f;
+
+// The points within rho of cell i -- REACH / 100 bins, less where the box of BOX
+// bins to every side ends before that or they are too many: position relative to i and half the squared distance
+// (3-D), or absolute and relative position (2-D).  Returns the number of
+// points, LOC + 1 or more if they do not fit.
+template <int D, int BOX, int REACH, int LOC>
+__device__ __forceinline__ unsigned gather_local(const Warp& w, const Grid& g, unsigned i, const Pt& pi, float4* p,
+                                                 unsigned* id, float& rho) {
+  const GridF& gf = g.f;
+  const float c[3] = {pi.x, pi.y, pi.z};
+  int b0[3] = {0, 0, 0}, b1[3] = {0, 0, 0};
+  rho = 1.0e9f;  // the box holds the whole grid
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const int b = bin1f(gf, d, c[d]);
+    b0[d] = imax(b - BOX, 0);
+    b1[d] = imin(b + BOX, gf.dims[d] - 1);
+    if (b0[d] > 0) rho = fminf(rho, c[d] - (gf.lo[d] + (float)b0[d] * gf.h) - 2.0f * gf.m);
+    if (b1[d] < gf.dims[d] - 1) rho = fminf(rho, gf.lo[d] + (float)(b1[d] + 1) * gf.h - c[d] - 2.0f * gf.m);
+  }
+  rho = fminf(rho, REACH * 0.01f * gf.h);
+  if (!(rho > 0.0f)) return (unsigned)LOC + 1u;
+  const int ny = b1[1] - b0[1] + 1, nz = b1[2] - b0[2] + 1;
+  unsigned n = 0u;
+  // a ball that holds too many points shrinks (twice at most)
+  for (int turn = 0; turn < 3; ++turn) {
+    const float rho2 = rho * rho;
+    n = 0u;
+    bool has = false;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    unsigned vid = 0u;
+    visit_rows(w, g, ny * nz, [&](int r, unsigned& lo, unsigned& hi) {
+      row_entries(g, b0[0], b1[0], b0[1] + r % ny, b0[2] + r / ny, lo, hi);
+    }, [&](unsigned e, const Pt& q) {
+      const float x = q.x - pi.x, y = q.y - pi.y, z = D >= 3 ? q.z - pi.z : 0.0f;
+      float d2 = x * x + y * y;
+      if (D >= 3) d2 = d2 + z * z;
+      has = e != i && d2 <= rho2;
+      v = D >= 3 ? make_float4(x, y, z, 0.5f * d2) : make_float4(q.x, q.y, x, y);
+      vid = e;
+      return true;
+    }, [&]() {
+      const unsigned m = w.ballot(has);
+      const unsigned at = n + (unsigned)__popc(m & ((1u << w.lane()) - 1u));
+      if (has && at < (unsigned)LOC) {
+        p[at] = v;
+        id[at] = vid;
+      }
+      n += (unsigned)__popc(m);
+      has = false;
+    });
+    if (n <= (unsigned)LOC) break;
+    const float f = 0.85f * (float)LOC / (float)n;
+    rho *= D >= 3 ? cbrtf(f) : sqrtf(f);
+  }
+  __syncwarp();
+  return n;
+}
+
+// One warp's working memory.
+template <int LOC>
+struct LocalScratch {
+  float4 p[LOC];
+  unsigned id[LOC];
+  unsigned short list[LOC];     // third points whose line may bound the face
+  ushort4 tet[160];             // 3-D: tetrahedra to verify (indices into p); z = kNoEnd: an open face, w its side
+  float4 cen[160];              // their centres (relative) and squared radii
+  unsigned rj[64], rr[64];      // partners and their counts
+};
+
+// Partners in ascending j to the cell's row.
+template <int LOC>
+__device__ __forceinline__ void write_row(const Warp& w, const LocalScratch<LOC>& sc, unsigned m, uint2* row, unsigned* len) {
+  __syncwarp();
+  for (unsigned e = w.lane(); e < m; e += 32u) {
+    const unsigned j = sc.rj[e];
+    unsigned rank = 0u;
+    for (unsigned k = 0; k < m; ++k) rank += sc.rj[k] < j ? 1u : 0u;
+    row[rank] = make_uint2(j, sc.rr[e]);
+  }
+  if (w.leader()) *len = m;
+}
+
+// The circumcentres of the listed tetrahedra, and whether every gathered point
+// lies outside their spheres with certainty.
+template <int LOC>
+__device__ __forceinline__ bool verify_tets(const Warp& w, const Grid& g, unsigned i, LocalScratch<LOC>& sc, unsigned n,
+                                            unsigned m) {
+  double pi[3];
+  load(g.P[i], pi);
+  bool bad = false;
+  for (unsigned t0 = 0; t0 < m; t0 += 32u) {
+    const unsigned t = t0 + w.lane();
+    const ushort4 q = sc.tet[t < m ? t : t0];
+    const bool closed = q.z != kNoEnd;
+    double a[3], b[3], c[3];
+    load(g.P[sc.id[q.x]], a);
+    load(g.P[sc.id[q.y]], b);
+    load(g.P[sc.id[closed ? q.z : q.x]], c);
+    double ha = 0.0, hb = 0.0, hc = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      a[d] -= pi[d];
+      b[d] -= pi[d];
+      c[d] -= pi[d];
+      ha += a[d] * a[d];
+      hb += b[d] * b[d];
+      hc += c[d] * c[d];
+    }
+    double bc[3], ca[3], ab[3];
+    cross3(b, c, bc);
+    cross3(c, a, ca);
+    cross3(a, b, ab);
+    const double inv = 0.5 / (a[0] * bc[0] + a[1] * bc[1] + a[2] * bc[2]);
+    const double xd[3] = {(ha * bc[0] + hb * ca[0] + hc * ab[0]) * inv, (ha * bc[1] + hb * ca[1] + hc * ab[1]) * inv,
+                          (ha * bc[2] + hb * ca[2] + hc * ab[2]) * inv};
+    const float x = (float)xd[0], y = (float)xd[1], z = (float)xd[2];
+    const float r2 = x * x + y * y + z * z;
+    if (t < m) sc.cen[t] = make_float4(x, y, z, r2);
+    if (closed && !(r2 < 1.0e12f)) bad = true;
+    const float m0 = kPowerX * r2;
+    for (unsigned k = 0; k < n; ++k) {
+      const float4 v = sc.p[k];
+      const float pw = v.w - (x * v.x + y * v.y + z * v.z);
+      if (closed && !(pw > kPowerV * v.w + m0) && k != q.x && k != q.y && k != q.z) {
+        // too near for float: once more in double
+        double pd[3], h = 0.0, dt = 0.0, xx = 0.0;
+        load(g.P[sc.id[k]], pd);
+        for (int d = 0; d < 3; ++d) {
+          pd[d] -= pi[d];
+          h += pd[d] * pd[d];
+          dt += pd[d] * xd[d];
+          xx += xd[d] * xd[d];
+        }
+        if (!(0.5 * h - dt > 1.0e-11 * (h + xx))) bad = true;
+      }
+    }
+    if (__any_sync(0xffffffffu, bad)) return false;
+  }
+  return true;
+}
+
+// Beyond the gathered ball: every cell outside the spheres that reach out of
+// it, and none on the open side of the open faces.  0: certain; 1: a cell
+// breaks one -- it joins the gathered points; 2: a cell is too near to tell,
+// or there is no room.
+template <int LOC>
+__device__ __forceinline__ int verify_far(const Warp& w, const Grid& g, unsigned i, LocalScratch<LOC>& sc, unsigned& n,
+                                          unsigned m, float rho) {
+  const Pt Pi = g.P[i];
+  const double pi[3] = {Pi.x, Pi.y, Pi.z};
+  int state = 0;
+  for (unsigned t = 0; t < m; ++t) {
+    const ushort4 q = sc.tet[t];
+    const float4 c = sc.cen[t];
+    const bool closed = q.z != kNoEnd;
+    if (closed && 4.0f * c.w <= rho * rho * 0.9999f) continue;
+    const unsigned ia = sc.id[q.x], ib = sc.id[q.y], ic = closed ? sc.id[q.z] : i;
+    const float4 va = sc.p[q.x], vb = sc.p[q.y];
+    float nx = va.y * vb.z - va.z * vb.y, ny = va.z * vb.x - va.x * vb.z, nz = va.x * vb.y - va.y * vb.x;
+    if (q.w == 2) { nx = -nx; ny = -ny; nz = -nz; }
+    // twice the rounding of n: 4 u |a| |b|
+    const float nm = 1.0e-6f * sqrtf(4.0f * va.w * vb.w);
+    bool hit = false, doubt = false;
+    unsigned hid = 0u;
+    float4 hv = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto test = [&](unsigned e, const Pt& p) {
+      if (e == i || e == ia || e == ib || e == ic) return true;
+      const float x = p.x - Pi.x, y = p.y - Pi.y, z = p.z - Pi.z;
+      const float h = 0.5f * (x * x + y * y + z * z);
+      const float lim = closed ? kPowerV * h + kPowerX * c.w : nm * sqrtf(2.0f * h);
+      const float pw = closed ? h - (c.x * x + c.y * y + c.z * z) : -(nx * x + ny * y + nz * z);
+      if (pw > lim) return true;
+      if (pw < -lim) hit = true;
+      else doubt = true;
+      hid = e;
+      hv = make_float4(x, y, z, h);
+      return false;
+    };
+    if (closed) {
+      const double cc[3] = {pi[0] + c.x, pi[1] + c.y, pi[2] + c.z};
+      visit_ball<3>(w, g, cc, (double)(sqrtf(c.w) * 1.0001f), test);
+    } else {
+      const double nn[3] = {nx, ny, nz};
+      visit_half<3>(w, g, pi, nn, test);
+    }
+    if (__any_sync(0xffffffffu, doubt)) return 2;
+    const unsigned b = __ballot_sync(0xffffffffu, hit);
+    if (b) {
+      const int src = __ffs(b) - 1;
+      hid = __shfl_sync(0xffffffffu, hid, src);
+      bool known = false;
+      for (unsigned k = w.lane(); k < n; k += 32u) known = known || sc.id[k] == hid;
+      state = 1;
+      if (!__any_sync(0xffffffffu, known)) {
+        if (n >= (unsigned)LOC) return 2;
+        if ((int)w.lane() == src) {
+          sc.p[n] = hv;
+          sc.id[n] = hid;
+        }
+        ++n;
+        __syncwarp();
+      }
+    }
+  }
+  return state;
+}
+
+// FAR: the spheres may reach out of the gathered ball and the cell may lie on
+// the hull; what lies beyond is looked up (verify_far), and cells that break a
+// sphere join the gathered points, until none does.
+template <int BOX, int REACH, int LOC, bool FAR>
+__device__ __forceinline__ bool cell_local3(const Warp& w, const Grid& g, unsigned i, LocalScratch<LOC>& sc, uint2* row,
+                                            unsigned* len) {
+  const unsigned lane = w.lane();
+  float rho;
+  unsigned n = gather_local<3, BOX, REACH, LOC>(w, g, i, g.P[i], sc.p, sc.id, rho);
+  if (n > (unsigned)LOC || n < 4u) return false;
+  if (!(rho * rho > g.rc2 * 1.0001f)) return false;
+  const float r2max = 0.25f * rho * rho;
+  const unsigned near_n = n;  // the in-cutoff cells are among the gathered ball's
+  for (int turn = 0; turn < 32; ++turn) {
+  unsigned rows = 0u, tets = 0u;
+  bool big = false;  // a sphere reaches out of the ball
+  for (unsigned t0 = 0; t0 < near_n; t0 += 32u) {
+    bool in = false;
+    if (t0 + lane < near_n) {
+      const float4 v = sc.p[t0 + lane];
+      float d2 = v.x * v.x + v.y * v.y;
+      d2 = d2 + v.z * v.z;
+      in = d2 < g.rc2;
+    }
+    for (unsigned bits = __ballot_sync(0xffffffffu, in); bits; bits &= bits - 1u) {
+      const unsigned J = t0 + (unsigned)__ffs(bits) - 1u;
+      const float4 vj = sc.p[J];
+      unsigned reps = 0u, members = 0u, mix = 0u;
+      // First the k whose triangle (i, j, k) has a circumradius below the
+      // largest sphere's, their lines cut off there.  Where these give no
+      // face, it is empty or lies farther out: then every gathered k, with its
+      // whole line; no interval means that the gathered points alone leave
+      // no face.
+      for (int wide = FAR ? 1 : 0; wide < 2 && members == 0u; ++wide) {
+        unsigned nk = 0u;
+        __syncwarp();
+        for (unsigned k0 = 0; k0 < n; k0 += 32u) {
+          const unsigned k = k0 + lane;
+          bool keep = false;
+          if (k < n && k != J) {
+            const float4 v = sc.p[k];
+            const float dt = vj.x * v.x + vj.y * v.y + vj.z * v.z;
+            const float jj = 2.0f * vj.w, kk = 2.0f * v.w;
+            const float w2 = jj * kk - dt * dt;
+            keep = wide || jj * kk * (jj + kk - 2.0f * dt) < 4.04f * r2max * w2 + 1.0e-5f * jj * kk * (jj + kk);
+          }
+          const unsigned b = __ballot_sync(0xffffffffu, keep);
+          if (keep) sc.list[nk + (unsigned)__popc(b & ((1u << lane) - 1u))] = (unsigned short)k;
+          nk += (unsigned)__popc(b);
+        }
+        __syncwarp();
+        float nearest_gap = -1.0e30f;
+        for (unsigned k0 = 0; k0 < nk; k0 += 32u) {
+          const bool act = k0 + lane < nk;
+          const unsigned k = act ? sc.list[k0 + lane] : J;
+          const float4 vk = sc.p[k];
+          const float wx = vj.y * vk.z - vj.z * vk.y, wy = vj.z * vk.x - vj.x * vk.z, wz = vj.x * vk.y - vj.y * vk.x;
+          const float w2 = wx * wx + wy * wy + wz * wz;
+          const float inv = 1.0f / w2;
+          // the circumcentre of (i, j, k) in their plane
+          const float x0 = (vj.w * (vk.y * wz - vk.z * wy) + vk.w * (wy * vj.z - wz * vj.y)) * inv;
+          const float y0 = (vj.w * (vk.z * wx - vk.x * wz) + vk.w * (wz * vj.x - wx * vj.z)) * inv;
+          const float z0 = (vj.w * (vk.x * wy - vk.y * wx) + vk.w * (wx * vj.y - wy * vj.x)) * inv;
+          const float room = 1.02f * r2max - (x0 * x0 + y0 * y0 + z0 * z0);
+          const bool alive = act && w2 > 0.0f && (wide || room > 0.0f);
+          float hi = !alive ? -1.0f : wide ? 1.0e15f : sqrtf(room * inv), lo = -hi;
+          unsigned hl = kNoEnd, ll = kNoEnd;
+          for (unsigned l0 = 0; l0 < n; l0 += 16u) {
+            if (!__any_sync(0xffffffffu, lo < hi)) break;
+            const unsigned l1 = min(l0 + 16u, n);
+#pragma unroll 4
+            for (unsigned l = l0; l < l1; ++l) {
+              if (l == J) continue;
+              const float4 v = sc.p[l];
+              const float wl = fmaf(wz, v.z, fmaf(wy, v.y, wx * v.x));
+              const float nm = v.w - fmaf(z0, v.z, fmaf(y0, v.y, x0 * v.x));
+              const float t = __fdividef(nm, wl);
+              if (l != k) {
+                if (wl > 0.0f && t < hi) { hi = t; hl = l; }
+                if (wl < 0.0f && t > lo) { lo = t; ll = l; }
+              }
+            }
+          }
+          const bool member = alive && lo < hi;
+          if (alive && !member) nearest_gap = fmaxf(nearest_gap, (hi - lo) * sqrtf(w2));
+          // an end at the largest sphere: its tetrahedron reaches out of the ball
+          if (!FAR && __any_sync(0xffffffffu, member && (wide || hl == kNoEnd || ll == kNoEnd))) return false;
+          members += (unsigned)__popc(__ballot_sync(0xffffffffu, member));
+          bool counted = false;
+          unsigned code = 0u;
+          if (member) {
+            if (hl != kNoEnd) {
+              counted = sc.id[hl] > sc.id[k];
+              code = (min(k, hl) << 16 | max(k, hl)) * 2654435761u;
+            }
+            if (ll != kNoEnd) {
+              counted = counted || sc.id[ll] > sc.id[k];
+              code ^= (min(k, ll) << 16 | max(k, ll)) * 2654435761u;
+            }
+          }
+          reps += (unsigned)__popc(__ballot_sync(0xffffffffu, counted));
+          mix ^= __reduce_xor_sync(0xffffffffu, code);
+          // each tetrahedron once, from its lesser third point
+#pragma unroll
+          for (int end = 0; end < 2; ++end) {
+            const unsigned l = end ? ll : hl;
+            const bool put = member && k < l;
+            const unsigned b = __ballot_sync(0xffffffffu, put);
+            const unsigned at = tets + (unsigned)__popc(b & ((1u << lane) - 1u));
+            if (put && at < 160u) 
+              sc.tet[at] = make_ushort4((unsigned short)J, (unsigned short)k, (unsigned short)l, (unsigned short)(end + 1));
+            tets += (unsigned)__popc(b);
+          }
+          if (tets > 160u) return false;
+        }
+        // no face: certain unless a line was missed by no more than the rounding
+        if (wide && members == 0u && __any_sync(0xffffffffu, nearest_gap > -3.0e-5f)) return false;
+      }
+      if (mix != 0u) return false;
+      if (reps) {
+        if (rows >= 64u) return false;
+        if (w.leader()) {
+          sc.rj[rows] = sc.id[J];
+          sc.rr[rows] = reps;
+        }
+        ++rows;
+      }
+      if (!FAR && tets > 96u) {
+        __syncwarp();
+        if (!verify_tets(w, g, i, sc, n, tets)) return false;
+        for (unsigned t = lane; t < tets; t += 32u)
+          if (!(4.0f * sc.cen[t].w <= rho * rho * 0.9999f)) big = true;
+        __syncwarp();
+        tets = 0u;
+      }
+    }
+  }
+  __syncwarp();
+  if (!verify_tets(w, g, i, sc, n, tets)) return false;
+  if (FAR) {
+    __syncwarp();
+    const int far = verify_far(w, g, i, sc, n, tets, rho);
+    if (far == 2) return false;
+    if (far == 1) continue;
+  } else {
+    for (unsigned t = lane; t < tets; t += 32u)
+      if (!(4.0f * sc.cen[t].w <= rho * rho * 0.9999f)) big = true;
+    if (__any_sync(0xffffffffu, big)) return false;
+  }
+  write_row(w, sc, rows, row, len);
+  return true;
+  }
+  return false;
+}
+
+
+template <int BOX, int REACH, int LOC>
+__device__ __forceinline__ bool cell_local2(const Warp& w, const Grid& g, unsigned i, LocalScratch<LOC>& sc, uint2* row,
+                                            unsigned* len) {
+  const unsigned lane = w.lane();
+  float rho;
+  const Pt Pi = g.P[i];
+  const unsigned n = gather_local<2, BOX, REACH, LOC>(w, g, i, Pi, sc.p, sc.id, rho);
+  if (n > (unsigned)LOC || n < 3u) return false;
+  if (!(rho * rho > g.rc2 * 1.0001f)) return false;
+  // the star: the circles through i and a with the least parameter on either
+  // side; those of an edge (or of one that the rounding may make an edge)
+  // have to lie within the disk with their tolerance
+  const float L0 = fmaxf(fabsf(Pi.x), fabsf(Pi.y));
+  bool bad = false;
+  unsigned edges = 0u;
+  for (unsigned a0 = 0; a0 < n; a0 += 32u) {
+    const bool act = a0 + lane < n;
+    const unsigned a = act ? a0 + lane : 0u;
+    const float4 va = sc.p[a];
+    const float a2 = va.z * va.z + va.w * va.w;
+    float left = 1.0e30f, right = -1.0e30f;
+    unsigned kl = kNoEnd, kr = kNoEnd;
+    for (unsigned q = 0; q < n; ++q) {
+      const float4 v = sc.p[q];
+      const float cr = va.z * v.w - va.w * v.z;
+      const float nm = (v.z * v.z + v.w * v.w) - (va.z * v.z + va.w * v.w);
+      const float s = __fdividef(nm, 2.0f * cr);
+      if (q != a) {
+        if (cr > 0.0f && s < left) { left = s; kl = q; }
+        if (cr < 0.0f && s > right) { right = s; kr = q; }
+      }
+    }
+    const bool edge = act && a2 > 0.0f && right <= left + 1.0e-3f * (1.0f + fabsf(left) + fabsf(right));
+    edges += (unsigned)__popc(__ballot_sync(0xffffffffu, edge));
+    if (edge) {
+      if (kl == kNoEnd || kr == kNoEnd) {
+        bad = true;
+      } else {
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+          const float s = side ? right : left;
+          const float4 vk = sc.p[side ? kr : kl];
+          const float R = a2 * (0.25f + s * s), r = sqrtf(R);
+          // shell_tol of the triangle (i, a, k), and the near test's slack
+          const float h2 = fmaxf(a2, vk.z * vk.z + vk.w * vk.w), hm = sqrtf(h2);
+          const float L = fmaxf(L0, fmaxf(fmaxf(fabsf(va.x), fabsf(va.y)), fmaxf(fabsf(vk.x), fabsf(vk.y))));
+          const float den = 2.0f * fabsf(va.z * vk.w - va.w * vk.z);
+          const float u = 0.5f * FLT_EPSILON;
+          const float dc = 48.0f * u * (L * L + h2) * hm / den + 8.0f * u * L;
+          const float tol = 1.01f * (4.0f * (2.0f * r * dc + dc * dc) + 32.0f * u * (R + L * r));
+          const float reach = sqrtf(R + tol);
+          const float slack = 1.0e-5f * (R + tol + 2.0f * reach * (2.0f * (L + r) + reach)) + 1.0e-30f;
+          if (!(1.01f * r + sqrtf(R + tol + slack) * 1.01f <= rho)) bad = true;
+          // the walk keeps at most kMaxNear points near a circle: a cell where
+          // it may drop some is the walk's
+          if (n >= (unsigned)kMaxNear) {
+            // centre relative to i: a / 2 + s (-a.y, a.x)
+            const float cx = 0.5f * va.z - s * va.w, cy = 0.5f * va.w + s * va.z;
+            const float lim = (R + tol + slack) * 1.01f;
+            unsigned near = 0u;
+            for (unsigned q = 0; q < n; ++q) {
+              const float e0 = sc.p[q].z - cx, e1 = sc.p[q].w - cy;
+              near += e0 * e0 + e1 * e1 <= lim ? 1u : 0u;
+            }
+            if (near >= (unsigned)kMaxNear) bad = true;
+          }
+        }
+      }
+    }
+  }
+  if (edges < 3u || __any_sync(0xffffffffu, bad)) return false;
+  const float li = sqlen2(Pi);
+  unsigned rows = 0u;
+  for (unsigned t0 = 0; t0 < n; t0 += 32u) {
+    bool in = false;
+    if (t0 + lane < n) {
+      const float4 v = sc.p[t0 + lane];
+      in = in_cutoff<2>(g, Pi, Pt{v.x, v.y, 0.0f, 0.0f});
+    }
+    for (unsigned bits = __ballot_sync(0xffffffffu, in); bits; bits &= bits - 1u) {
+      const unsigned J = t0 + (unsigned)__ffs(bits) - 1u;
+      const Pt pj{sc.p[J].x, sc.p[J].y, 0.0f, 0.0f};
+      const float lj = sqlen2(pj);
+      unsigned reps = 0u;
+      for (unsigned k0 = 0; k0 < n; k0 += 32u) {
+        const unsigned k = k0 + lane;
+        bool open = k < n && k != J;
+        float c[2] = {0.f, 0.f}, r2 = 0.f;
+        if (open) {
+          // naive_delaunay.hpp:62-99, as tri_pass
+          const Pt pk{sc.p[k].x, sc.p[k].y, 0.0f, 0.0f};
+          const float den = 2.0f * (Pi.x * (pj.y - pk.y) + pj.x * (pk.y - Pi.y) + pk.x * (Pi.y - pj.y));
+          open = !(fabsf(den) <= FLT_EPSILON);
+          const float lk = sqlen2(pk);
+          c[0] = (li * (pj.y - pk.y) + lj * (pk.y - Pi.y) + lk * (Pi.y - pj.y)) / den;
+          c[1] = (li * (pk.x - pj.x) + lj * (Pi.x - pk.x) + lk * (pj.x - Pi.x)) / den;
+          const float e0 = Pi.x - c[0], e1 = Pi.y - c[1];
+          r2 = e0 * e0 + e1 * e1;
+        }
+        for (unsigned m0 = 0; m0 < n; m0 += 8u) {
+          if (!__any_sync(0xffffffffu, open)) break;
+          const unsigned m1 = min(m0 + 8u, n);
+          for (unsigned m = m0; m < m1; ++m) {
+            const float4 v = sc.p[m];
+            const float f0 = v.x - c[0], f1 = v.y - c[1];
+            if (f0 * f0 + f1 * f1 <= r2 && m != J && m != k) open = false;
+          }
+        }
+        // a circle without a gathered point has to lie within the disk
+        const float r = sqrtf(r2);
+        if (__any_sync(0xffffffffu, open && !(2.0f * r * 1.00001f <= rho))) return false;
+        reps += (unsigned)__popc(__ballot_sync(0xffffffffu, open));
+      }
+      if (reps) {
+        if (rows >= 64u) return false;
+        if (w.leader()) {
+          sc.rj[rows] = sc.id[J];
+          sc.rr[rows] = reps;
+        }
+        ++rows;
+      }
+    }
+  }
+  write_row(w, sc, rows, row, len);
+  return true;
+}
+
+template <int D, int BOX, int REACH, int LOC, bool FAR>
+__device__ __forceinline__ bool cell_local(const Warp& w, const Grid& g, unsigned i, LocalScratch<LOC>& sc, uint2* row,
+                                           unsigned* len) {
+  if (D == 3) return cell_local3<BOX, REACH, LOC, FAR>(w, g, i, sc, row, len);
+  return cell_local2<BOX, REACH, LOC>(w, g, i, sc, row, len);
+}
+
+}  // namespace dl
+}  // namespace tecs

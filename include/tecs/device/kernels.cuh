@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "forces.cuh"
 #include "delaunay_star.cuh"
+#include "delaunay_local.cuh"
 
 namespace tecs {
 
@@ -734,6 +735,10 @@ struct DlState {
   double h, inv;
   int dims[3];
   unsigned nbins;
+  dl::GridF f;
+  // cells handed on by the local search's levels, and the cells taken from
+  // each list so far
+  unsigned left[2], taken[3];
 };
 
 __device__ __forceinline__ unsigned f2ord(float f) {
@@ -745,7 +750,12 @@ __device__ __forceinline__ float ord2f(unsigned u) {
 }
 
 static __global__ void k_dl_reset(DlState* st) {
-  if (threadIdx.x < 3) { st->mm[threadIdx.x] = 0xffffffffu; st->mm[3 + threadIdx.x] = 0u; }
+  if (threadIdx.x < 3) {
+    st->mm[threadIdx.x] = 0xffffffffu;
+    st->mm[3 + threadIdx.x] = 0u;
+    st->taken[threadIdx.x] = 0u;
+    if (threadIdx.x < 2) st->left[threadIdx.x] = 0u;
+  }
 }
 
 template <int D>
@@ -785,6 +795,7 @@ static __global__ void k_dl_plan(const Counters* __restrict__ ctr, unsigned max_
   st->h = g.h;
   st->inv = g.inv;
   st->nbins = g.nbins;
+  st->f = g.f;
 }
 
 __device__ __forceinline__ dl::Grid dl_view(const DlState* st) {
@@ -793,6 +804,7 @@ __device__ __forceinline__ dl::Grid dl_view(const DlState* st) {
   g.h = st->h;
   g.inv = st->inv;
   g.nbins = st->nbins;
+  g.f = st->f;
   return g;
 }
 
@@ -855,36 +867,87 @@ static __global__ void k_dl_scatter(const float4* __restrict__ X, const Counters
   sp[at] = v;
 }
 
-// one warp per cell: the lanes share each search's entries (dl::Warp)
-template <int D>
-static __global__ void __launch_bounds__(kDlThreads) k_dl_mult(const float4* __restrict__ X, Counters* __restrict__ ctr,
-                                                               const DlState* __restrict__ st,
-                                                               const unsigned* __restrict__ off,
-                                                               const unsigned* __restrict__ idx,
-                                                               const float4* __restrict__ sp, float rc2,
-                                                               uint2* __restrict__ row, unsigned* __restrict__ len) {
-  const unsigned n = ctr->n;
-  const unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // the same in every lane of the warp
-  if (i >= n) return;
+__device__ __forceinline__ dl::Grid dl_grid(const float4* X, const Counters* ctr, const DlState* st, const unsigned* off,
+                                            const unsigned* idx, const float4* sp, float rc2) {
   dl::Grid g = dl_view(st);
   g.off = off;
   g.idx = idx;
   g.sp = reinterpret_cast<const dl::Pt*>(sp);
   g.P = reinterpret_cast<const dl::Pt*>(X);
-  g.n = n;
+  g.n = ctr->n;
   g.rc2 = rc2;
+  return g;
+}
+
+// The local search (delaunay_local.cuh), one warp per cell.  LEVEL 0: every
+// cell, in bin order; LEVEL 1: the cells that level 0 handed on, in 2-D over a
+// larger box, in 3-D looking up what lies beyond the gathered ball.  The cells
+// that a level is not certain of go to its list.
+// Radii: 1.75 bins hold about 85 points in a ball of cells (two cells a bin of
+// its bounding box), enough for 97 % of the interior cells (spheres of 1.4 cell
+// spacings); in 2-D 2.25 bins hold about 40, enough for all but the hull.
+template <int D, int LEVEL>
+static __global__ void __launch_bounds__(dl::kLocalThreads)
+    k_dl_local(const float4* __restrict__ X, const Counters* __restrict__ ctr, DlState* __restrict__ st,
+               const unsigned* __restrict__ off, const unsigned* __restrict__ idx, const float4* __restrict__ sp,
+               float rc2, uint2* __restrict__ row, unsigned* __restrict__ len, const unsigned* __restrict__ in,
+               unsigned* __restrict__ out) {
+  constexpr int BOX = LEVEL == 1 && D == 2 ? 4 : 2;
+  constexpr int REACH = D == 3 ? 175 : (LEVEL == 0 ? 225 : 450);
+  constexpr int LOC = LEVEL == 0 ? 112 : (D == 3 ? 192 : 320);
+  __shared__ dl::LocalScratch<LOC> scratch[dl::kLocalThreads / 32];
+  dl::LocalScratch<LOC>& sc = scratch[threadIdx.x >> 5];
+  const dl::Grid g = dl_grid(X, ctr, st, off, idx, sp, rc2);
+  const dl::Warp lanes;
+  const unsigned count = LEVEL == 0 ? g.n : st->left[0];
+  for (;;) {
+    unsigned at = 0u;
+    if (lanes.leader()) at = atomicAdd(&st->taken[LEVEL], 1u);
+    at = lanes.bcast(at, 0);
+    if (at >= count) return;
+    const unsigned i = in[at];
+    __syncwarp();
+    if (!dl::cell_local<D, BOX, REACH, LOC, LEVEL == 1>(lanes, g, i, sc, row + (size_t)i * kDlRow, len + i) && lanes.leader())
+      out[atomicAdd(&st->left[LEVEL], 1u)] = i;
+    __syncwarp();
+  }
+}
+
+// The cells that the local search was not certain of: the walk in double, one
+// warp per cell, the lanes sharing each search's entries (dl::Warp).
+template <int D>
+static __global__ void __launch_bounds__(kDlThreads) k_dl_mult(const float4* __restrict__ X, Counters* __restrict__ ctr,
+                                                               DlState* __restrict__ st,
+                                                               const unsigned* __restrict__ off,
+                                                               const unsigned* __restrict__ idx,
+                                                               const float4* __restrict__ sp, float rc2,
+                                                               uint2* __restrict__ row, unsigned* __restrict__ len,
+                                                               const unsigned* __restrict__ in) {
   // the warp's star and candidate lists: one copy, in shared memory
   __shared__ __align__(16) unsigned char scratch[(kDlThreads / 32) * sizeof(dl::Scratch)];
   dl::Scratch& sc = reinterpret_cast<dl::Scratch*>(scratch)[threadIdx.x >> 5];
-  unsigned oj[kDlRow], orp[kDlRow], err = 0;
+  __shared__ unsigned out_j[kDlThreads / 32][kDlRow], out_r[kDlThreads / 32][kDlRow];
+  unsigned *oj = out_j[threadIdx.x >> 5], *orp = out_r[threadIdx.x >> 5];
+  const dl::Grid g = dl_grid(X, ctr, st, off, idx, sp, rc2);
   const dl::Warp lanes;
-  const unsigned m = dl::cell_mult<D>(lanes, g, i, oj, orp, kDlRow, &err, sc);
-  if (lanes.lane() != 0u) return;
-  for (unsigned t = 0; t < m; ++t) row[(size_t)i * kDlRow + t] = make_uint2(oj[t], orp[t]);
-  len[i] = m;
-  // a full near-circle list keeps the points nearest the circle (no error);
-  // any other overflow leaves the row incomplete
-  if (err & (dl::kErrStar | dl::kErrPairs | dl::kErrList)) atomicOr(&ctr->error, 4u);
+  const unsigned count = st->left[1];
+  for (;;) {
+    unsigned at = 0u;
+    if (lanes.leader()) at = atomicAdd(&st->taken[2], 1u);
+    at = lanes.bcast(at, 0);
+    if (at >= count) return;
+    const unsigned i = in[at];
+    unsigned err = 0;
+    const unsigned m = dl::cell_mult<D>(lanes, g, i, oj, orp, kDlRow, &err, sc);
+    for (unsigned t = lanes.lane(); t < m; t += 32u) row[(size_t)i * kDlRow + t] = make_uint2(oj[t], orp[t]);
+    __syncwarp();
+    if (lanes.leader()) {
+      len[i] = m;
+      // a full near-circle list keeps the points nearest the circle (no error);
+      // any other overflow leaves the row incomplete
+      if (err & (dl::kErrStar | dl::kErrPairs | dl::kErrList)) atomicOr(&ctr->error, 4u);
+    }
+  }
 }
 
 template <int D, int FINDER, int FORCE>

@@ -192,6 +192,7 @@ struct tecs_sim {
   // sorted slots and positions) and each cell's partner row
   DlState* dl_st = nullptr;
   unsigned *dl_cnt = nullptr, *dl_off = nullptr, *dl_idx = nullptr, *dl_len = nullptr;
+  unsigned* dl_list = nullptr;  // cells handed on by the local search's levels, capacity each
   float4* dl_sp = nullptr;
   uint2* dl_row = nullptr;
   unsigned dl_maxbins = 0;
@@ -445,6 +446,9 @@ int enqueue_rebuild(tecs_sim* s, int& K, bool run_count) {
   return 0;
 }
 
+// Blocks of the Delaunay finder's searches: 8 an SM.
+constexpr unsigned kDlBlocks = 152 * 8;
+
 // The Delaunay finder of any capacity: bin grid of the pass's positions, then
 // every cell's partner row.
 int enqueue_delaunay_star(tecs_sim* s, const PassArgs& a, int& K) {
@@ -465,14 +469,28 @@ int enqueue_delaunay_star(tecs_sim* s, const PassArgs& a, int& K) {
   else k_dl_scatter<2><<<gb, 256, 0, s->stream>>>(a.X, s->ctr, s->dl_st, s->dl_cnt, s->dl_off, s->dl_idx, s->dl_sp);
   PROF_END(s, "k_dl_grid");
   K += 6;
-  const unsigned mb = ceil_div(L ? L : 1, kDlThreads / 32);  // one warp per cell
+  // warps take cells from the lists until none is left: at most as many blocks
+  // as the cells need, or as the GPU holds
+  const unsigned lb = std::min(ceil_div(L ? L : 1, dl::kLocalThreads / 32), kDlBlocks);
+  const unsigned mb = std::min(ceil_div(L ? L : 1, kDlThreads / 32), kDlBlocks);
+  unsigned *l0 = s->dl_list, *l1 = l0 + s->d.capacity;
+#define DL_PASS(DD)                                                                                                  \
+  k_dl_local<DD, 0><<<lb, dl::kLocalThreads, 0, s->stream>>>(a.X, s->ctr, s->dl_st, s->dl_off, s->dl_idx, s->dl_sp,  \
+                                                             s->fp.rc2, s->dl_row, s->dl_len, s->dl_idx, l0);        \
+  PROF_END(s, "k_dl_local");                                                                                         \
+  PROF_BEGIN(s);                                                                                                     \
+  k_dl_local<DD, 1><<<lb, dl::kLocalThreads, 0, s->stream>>>(a.X, s->ctr, s->dl_st, s->dl_off, s->dl_idx, s->dl_sp,  \
+                                                             s->fp.rc2, s->dl_row, s->dl_len, l0, l1);               \
+  PROF_END(s, "k_dl_local_far");                                                                                     \
+  PROF_BEGIN(s);                                                                                                     \
+  k_dl_mult<DD><<<mb, kDlThreads, 0, s->stream>>>(a.X, s->ctr, s->dl_st, s->dl_off, s->dl_idx, s->dl_sp, s->fp.rc2,  \
+                                                  s->dl_row, s->dl_len, l1);                                         \
+  PROF_END(s, "k_dl_mult")
   PROF_BEGIN(s);
-  if (d3) k_dl_mult<3><<<mb, kDlThreads, 0, s->stream>>>(a.X, s->ctr, s->dl_st, s->dl_off, s->dl_idx, s->dl_sp,
-                                                         s->fp.rc2, s->dl_row, s->dl_len);
-  else k_dl_mult<2><<<mb, kDlThreads, 0, s->stream>>>(a.X, s->ctr, s->dl_st, s->dl_off, s->dl_idx, s->dl_sp,
-                                                      s->fp.rc2, s->dl_row, s->dl_len);
-  PROF_END(s, "k_dl_mult");
-  K += 1;
+  if (d3) { DL_PASS(3); }
+  else { DL_PASS(2); }
+#undef DL_PASS
+  K += 3;
   CK(cudaGetLastError());
   return 0;
 }
@@ -892,7 +910,7 @@ int tecs_sim_create(const tecs_sim_desc* desc, tecs_sim** out) {
     ok = ok && alloc((void**)&s->dl_st, sizeof(DlState)) && alloc((void**)&s->dl_cnt, (size_t)s->dl_maxbins * 4) &&
          alloc((void**)&s->dl_off, ((size_t)s->dl_maxbins + 1) * 4) && alloc((void**)&s->dl_idx, cap * 4) &&
          alloc((void**)&s->dl_sp, cap * 16) && alloc((void**)&s->dl_row, cap * kDlRow * 8) &&
-         alloc((void**)&s->dl_len, cap * 4);
+         alloc((void**)&s->dl_len, cap * 4) && alloc((void**)&s->dl_list, 2 * cap * 4);
     if (ok) ok = cudaMemsetAsync(s->dl_len, 0, cap * 4, s->stream) == cudaSuccess;
   }
   if (s->binned) {
@@ -931,7 +949,7 @@ int tecs_sim_destroy(tecs_sim* s) {
   void* ptrs[] = {s->A, s->B, s->Xt, s->d1, s->d2, s->PA, s->PB, s->Pt, s->dp1, s->dp2, s->key, s->rank, s->src,
                   s->cnt, s->off, s->part, s->div_parent, s->div_slot, s->ctr, s->com_part, s->com, s->stage,
                   s->Bid, s->dmult, s->link_off, s->link_ent, s->slot_of, s->ov, s->EA, s->EB, s->Et,
-                  s->ed1, s->ed2, s->dl_st, s->dl_cnt, s->dl_off, s->dl_idx, s->dl_sp, s->dl_row, s->dl_len};
+                  s->ed1, s->ed2, s->dl_st, s->dl_cnt, s->dl_off, s->dl_idx, s->dl_sp, s->dl_row, s->dl_len, s->dl_list};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (s->stream) cudaStreamDestroy(s->stream);
