@@ -31,8 +31,9 @@
 //
 // What bounds it: instruction issue, then the latency of the few cells left to
 // the walk.  40k cells in space, one pass: 54 ms (the walk for every cell) ->
-// 3.3 (1.4 the first search, 0.9 the second over 7 % of the cells, 0.8 the
-// walk of 9 cells); 30k in the plane, two passes: 32 -> 3.7 ms.
+// 2.3-2.8 (0.9 the first search, 0.9-1.3 the second over 7 % of the cells,
+// 0-0.8 the walk of at most 9 cells); 30k in the plane, two passes: 27-32 ->
+// 3.3-3.7 ms.
 #pragma once
 
 #include "delaunay_star.cuh"
@@ -130,6 +131,70 @@ __device__ __forceinline__ void write_row(const Warp& w, const LocalScratch<LOC>
   if (w.leader()) *len = m;
 }
 
+// The gathered points put in order of their distance, by eighths of rho^2: a
+// search may stop where every later point is too far (the first search of 40k
+// cells 1.4 -> 0.9 ms).
+constexpr int kShells = 8;
+template <int LOC>
+__device__ __forceinline__ void order_points(const Warp& w, LocalScratch<LOC>& sc, unsigned n, float rho) {
+  constexpr int C = (LOC + 31) / 32;
+  float4 v[C];
+  unsigned id[C], to[C];
+  const float inv = (float)kShells / (rho * rho);
+  unsigned base = 0u;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const unsigned k = 32u * c + w.lane();
+    v[c] = sc.p[k < n ? k : 0u];
+    id[c] = sc.id[k < n ? k : 0u];
+    to[c] = 0u;
+  }
+  for (int s = 0; s < kShells; ++s) {
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const unsigned k = 32u * c + w.lane();
+      const bool here = k < n && min((int)(2.0f * v[c].w * inv), kShells - 1) == s;
+      const unsigned b = __ballot_sync(0xffffffffu, here);
+      if (here) to[c] = base + (unsigned)__popc(b & ((1u << w.lane()) - 1u));
+      base += (unsigned)__popc(b);
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    if (32u * c + w.lane() < n) {
+      sc.p[to[c]] = v[c];
+      sc.id[to[c]] = id[c];
+    }
+  __syncwarp();
+}
+
+// The circumcentre of the cell at pi and three others, relative to the cell.
+__device__ __forceinline__ void tet_centre(const Grid& g, const double* pi, unsigned ia, unsigned ib, unsigned ic,
+                                           double* x) {
+  double a[3], b[3], c[3];
+  load(g.P[ia], a);
+  load(g.P[ib], b);
+  load(g.P[ic], c);
+  double ha = 0.0, hb = 0.0, hc = 0.0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    a[d] -= pi[d];
+    b[d] -= pi[d];
+    c[d] -= pi[d];
+    ha += a[d] * a[d];
+    hb += b[d] * b[d];
+    hc += c[d] * c[d];
+  }
+  double bc[3], ca[3], ab[3];
+  cross3(b, c, bc);
+  cross3(c, a, ca);
+  cross3(a, b, ab);
+  const double inv = 0.5 / (a[0] * bc[0] + a[1] * bc[1] + a[2] * bc[2]);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) x[d] = (ha * bc[d] + hb * ca[d] + hc * ab[d]) * inv;
+}
+
 // The circumcentres of the listed tetrahedra, and whether every gathered point
 // lies outside their spheres with certainty.
 template <int LOC>
@@ -142,27 +207,8 @@ __device__ __forceinline__ bool verify_tets(const Warp& w, const Grid& g, unsign
     const unsigned t = t0 + w.lane();
     const ushort4 q = sc.tet[t < m ? t : t0];
     const bool closed = q.z != kNoEnd;
-    double a[3], b[3], c[3];
-    load(g.P[sc.id[q.x]], a);
-    load(g.P[sc.id[q.y]], b);
-    load(g.P[sc.id[closed ? q.z : q.x]], c);
-    double ha = 0.0, hb = 0.0, hc = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      a[d] -= pi[d];
-      b[d] -= pi[d];
-      c[d] -= pi[d];
-      ha += a[d] * a[d];
-      hb += b[d] * b[d];
-      hc += c[d] * c[d];
-    }
-    double bc[3], ca[3], ab[3];
-    cross3(b, c, bc);
-    cross3(c, a, ca);
-    cross3(a, b, ab);
-    const double inv = 0.5 / (a[0] * bc[0] + a[1] * bc[1] + a[2] * bc[2]);
-    const double xd[3] = {(ha * bc[0] + hb * ca[0] + hc * ab[0]) * inv, (ha * bc[1] + hb * ca[1] + hc * ab[1]) * inv,
-                          (ha * bc[2] + hb * ca[2] + hc * ab[2]) * inv};
+    double xd[3];
+    tet_centre(g, pi, sc.id[q.x], sc.id[q.y], sc.id[closed ? q.z : q.x], xd);
     const float x = (float)xd[0], y = (float)xd[1], z = (float)xd[2];
     const float r2 = x * x + y * y + z * z;
     if (t < m) sc.cen[t] = make_float4(x, y, z, r2);
@@ -210,30 +256,63 @@ __device__ __forceinline__ int verify_far(const Warp& w, const Grid& g, unsigned
     if (q.w == 2) { nx = -nx; ny = -ny; nz = -nz; }
     // twice the rounding of n: 4 u |a| |b|
     const float nm = 1.0e-6f * sqrtf(4.0f * va.w * vb.w);
-    bool hit = false, doubt = false;
+    bool hit = false;
     unsigned hid = 0u;
     float4 hv = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto test = [&](unsigned e, const Pt& p) {
-      if (e == i || e == ia || e == ib || e == ic) return true;
-      const float x = p.x - Pi.x, y = p.y - Pi.y, z = p.z - Pi.z;
-      const float h = 0.5f * (x * x + y * y + z * z);
-      const float lim = closed ? kPowerV * h + kPowerX * c.w : nm * sqrtf(2.0f * h);
-      const float pw = closed ? h - (c.x * x + c.y * y + c.z * z) : -(nx * x + ny * y + nz * z);
-      if (pw > lim) return true;
-      if (pw < -lim) hit = true;
-      else doubt = true;
-      hid = e;
-      hv = make_float4(x, y, z, h);
-      return false;
-    };
-    if (closed) {
-      const double cc[3] = {pi[0] + c.x, pi[1] + c.y, pi[2] + c.z};
-      visit_ball<3>(w, g, cc, (double)(sqrtf(c.w) * 1.0001f), test);
-    } else {
-      const double nn[3] = {nx, ny, nz};
-      visit_half<3>(w, g, pi, nn, test);
+    // in float, and where a cell is too near to tell, once more in double
+    for (int dbl = 0; dbl < 2; ++dbl) {
+      bool doubt = false;
+      double xd[3] = {0.0, 0.0, 0.0}, xx = 0.0;
+      if (dbl && closed) {
+        tet_centre(g, pi, ia, ib, ic, xd);
+        xx = xd[0] * xd[0] + xd[1] * xd[1] + xd[2] * xd[2];
+      } else if (dbl) {
+        double a[3], b[3];
+        load(g.P[ia], a);
+        load(g.P[ib], b);
+        for (int d = 0; d < 3; ++d) { a[d] -= pi[d]; b[d] -= pi[d]; }
+        cross3(a, b, xd);
+        if (q.w == 2)
+          for (int d = 0; d < 3; ++d) xd[d] = -xd[d];
+        xx = sqrt((a[0] * a[0] + a[1] * a[1] + a[2] * a[2]) * (b[0] * b[0] + b[1] * b[1] + b[2] * b[2]));
+      }
+      auto test = [&](unsigned e, const Pt& p) {
+        if (e == i || e == ia || e == ib || e == ic) return true;
+        const float x = p.x - Pi.x, y = p.y - Pi.y, z = p.z - Pi.z;
+        const float h = 0.5f * (x * x + y * y + z * z);
+        bool out, in;
+        if (!dbl) {
+          const float lim = closed ? kPowerV * h + kPowerX * c.w : nm * sqrtf(2.0f * h);
+          const float pw = closed ? h - (c.x * x + c.y * y + c.z * z) : -(nx * x + ny * y + nz * z);
+          out = pw > lim;
+          in = pw < -lim;
+        } else {
+          const double v[3] = {p.x - pi[0], p.y - pi[1], p.z - pi[2]};
+          const double vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+          const double dt = v[0] * xd[0] + v[1] * xd[1] + v[2] * xd[2];
+          const double pw = closed ? 0.5 * vv - dt : -dt;
+          const double lim = closed ? 1.0e-11 * (vv + xx) : 1.0e-13 * xx * sqrt(vv);
+          out = pw > lim;
+          in = pw < -lim;
+        }
+        if (out) return true;
+        hit = in;
+        doubt = !in;
+        hid = e;
+        hv = make_float4(x, y, z, h);
+        return false;
+      };
+      if (closed) {
+        const double cc[3] = {pi[0] + c.x, pi[1] + c.y, pi[2] + c.z};
+        visit_ball<3>(w, g, cc, (double)(sqrtf(c.w) * 1.0001f), test);
+      } else {
+        const double nn[3] = {nx, ny, nz};
+        visit_half<3>(w, g, pi, nn, test);
+      }
+      if (!__any_sync(0xffffffffu, doubt)) break;
+      if (dbl) return 2;
+      hit = false;
     }
-    if (__any_sync(0xffffffffu, doubt)) return 2;
     const unsigned b = __ballot_sync(0xffffffffu, hit);
     if (b) {
       const int src = __ffs(b) - 1;
@@ -266,6 +345,8 @@ __device__ __forceinline__ bool cell_local3(const Warp& w, const Grid& g, unsign
   unsigned n = gather_local<3, BOX, REACH, LOC>(w, g, i, g.P[i], sc.p, sc.id, rho);
   if (n > (unsigned)LOC || n < 4u) return false;
   if (!(rho * rho > g.rc2 * 1.0001f)) return false;
+  order_points(w, sc, n, rho);
+  const float shell = rho * rho / (float)kShells;
   const float r2max = 0.25f * rho * rho;
   const unsigned near_n = n;  // the in-cutoff cells are among the gathered ball's
   for (int turn = 0; turn < 32; ++turn) {
@@ -322,9 +403,18 @@ __device__ __forceinline__ bool cell_local3(const Warp& w, const Grid& g, unsign
           const bool alive = act && w2 > 0.0f && (wide || room > 0.0f);
           float hi = !alive ? -1.0f : wide ? 1.0e15f : sqrtf(room * inv), lo = -hi;
           unsigned hl = kNoEnd, ll = kNoEnd;
-          for (unsigned l0 = 0; l0 < n; l0 += 16u) {
-            if (!__any_sync(0xffffffffu, lo < hi)) break;
-            const unsigned l1 = min(l0 + 16u, n);
+          for (unsigned l0 = 0; l0 < n;) {
+            // a point cuts an interval only from within twice its ends' distance
+            // to the cell; the points come in shells of growing distance
+            const float end = fmaxf(hi, -lo);
+            const float r2 = lo < hi ? x0 * x0 + y0 * y0 + z0 * z0 + end * end * w2 : 0.0f;
+            const float far2 = 4.001f * __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(r2)));
+            if (far2 == 0.0f) break;
+            if (l0 < near_n && floorf(2.0f * sc.p[l0].w / shell * 0.99999f) * shell > far2) {
+              l0 = near_n;  // only points looked up from beyond the ball are left
+              if (l0 >= n) break;
+            }
+            const unsigned l1 = min(l0 + 8u, l0 < near_n ? near_n : n);
 #pragma unroll 4
             for (unsigned l = l0; l < l1; ++l) {
               if (l == J) continue;
@@ -337,6 +427,7 @@ __device__ __forceinline__ bool cell_local3(const Warp& w, const Grid& g, unsign
                 if (wl < 0.0f && t > lo) { lo = t; ll = l; }
               }
             }
+            l0 = l1;
           }
           const bool member = alive && lo < hi;
           if (alive && !member) nearest_gap = fmaxf(nearest_gap, (hi - lo) * sqrtf(w2));
