@@ -229,8 +229,9 @@ static __global__ void k_scan_reduce(const unsigned* __restrict__ cnt, unsigned 
   unsigned t = block_sum(v, sh);
   if (threadIdx.x == 0) {
     part[blockIdx.x] = t;
-    // the super sums follow the chunk partials and are zeroed before this kernel
-    atomicAdd(&part[gridDim.x + blockIdx.x / kScanSuper], t);
+    // the super sums follow the chunk partials; k_scan_apply reads them past the
+    // first kScanSuper chunks only, and only then they are zeroed before this kernel
+    if (gridDim.x > kScanSuper) atomicAdd(&part[gridDim.x + blockIdx.x / kScanSuper], t);
   }
 }
 
@@ -1137,10 +1138,16 @@ __device__ __forceinline__ void pass_epilogue(const GridP& g, const PassArgs& a,
 // than kMaxNb neighbours takes the general path.
 constexpr int kMaxNb = 24;     // (4 on average at one cell per bin, 12 in packed tissue; a count is a class: at most 31)
 constexpr int kPool = 224;     // neighbours of a warp's cells at a time (about 130 at one cell per bin)
-// Threads (cells) per block of the cooperative passes: three warps.  The
-// block's shared memory (about 24 KB) then lets nine blocks share an SM, 864
-// cells, so that a 100k-cell pass runs in a single wave on 152 SMs.
+// Threads (cells) per block of the passes; of the cooperative pass over the
+// grid by the law: the spring laws four warps at 72 registers, so that seven
+// blocks (28 warps) share an SM (at 96 threads and nine blocks 136 us a pass of
+// 1M cells, here 126; at 64 and 32 threads 138 and 150); the polarity law three
+// warps, seven blocks (21 warps at 96 registers): a 100k-cell pass runs in a
+// single wave on 152 SMs (six blocks: 53 us, seven 44, four warps 47 to 49).
 constexpr int kPassThreads = 96;
+template <int FORCE>
+constexpr int kCoopThreads = FORCE == 2 ? 96 : 128;
+constexpr int kCoopBlocks = 7;  // an SM
 // Position arrays that the cooperative pass scans hold this many float4 past
 // their capacity: the candidate scan reads rounds of four places past a
 // list's end and leaves their bits out.
@@ -1587,11 +1594,11 @@ struct BallBins {
     if (s_ < a.pair_cap)                                                                      \
       a.pairs[s_] = make_uint2(id_at(a.X, a.Bid, i - (unsigned)lane + (c)), id_at(a.X, a.Bid, (jj))); \
   }
-#define TECS_PASS_BODY(BLK)                                                                   \
+#define TECS_PASS_BODY(BLK, THREADS)                                                          \
   static_assert(FORCE <= 1 || (FORCE == 2 && D == 3), "spring laws, or the 3-D polarity law"); \
   static_assert(FINDER == 1 || FINDER == 3, "the binned finders");                            \
   constexpr bool POL = FORCE == 2;                                                            \
-  constexpr int TB = kPassThreads;                                                            \
+  constexpr int TB = (THREADS);                                                               \
   const unsigned n = a.ctr->n;                                                                \
   const unsigned i = (BLK)*TB + threadIdx.x;                                                  \
   const bool run = i < n;                                                                     \
@@ -1618,8 +1625,9 @@ struct BallBins {
 
 // The grid pass: block blockIdx.x's cells.
 template <int D, int FORCE, int FINDER = 3>
-static __global__ void __launch_bounds__(kPassThreads, FORCE == 2 ? 6 : 9) k_pass_gabriel(GridP g, ForceP fp, PassArgs a) {
-  TECS_PASS_BODY(blockIdx.x)
+static __global__ void __launch_bounds__(kCoopThreads<FORCE>, kCoopBlocks)
+    k_pass_gabriel(GridP g, ForceP fp, PassArgs a) {
+  TECS_PASS_BODY(blockIdx.x, kCoopThreads<FORCE>)
 #include "pass_gabriel_body.inc"
   TECS_PASS_END
 }
@@ -1629,7 +1637,7 @@ static __global__ void __launch_bounds__(kPassThreads, FORCE == 2 ? 6 : 9) k_pas
 template <int D, int FORCE, int FINDER = 3>
 __device__ __forceinline__ void pass_gabriel_block(const GridP& g, const ForceP& fp, const PassArgs& a,
                                                    const unsigned blk) {
-  TECS_PASS_BODY(blk)
+  TECS_PASS_BODY(blk, kPassThreads)
 #include "pass_gabriel_body.inc"
   TECS_PASS_END
 }

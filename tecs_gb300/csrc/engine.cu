@@ -159,7 +159,7 @@ static __global__ void k_eorder_gather(const unsigned* __restrict__ off, unsigne
 #define TECS_CAPTURE(c, jj)
 
 template <int PASS, bool POL, int TB>
-static __global__ void __launch_bounds__(TB, (POL ? 576 : 864) / TB) k_epass(EngArgs e) {
+static __global__ void __launch_bounds__(TB, (POL ? 672 : 896) / TB) k_epass(EngArgs e) {
   constexpr int D = 3;
   __shared__ unsigned hsim[TB];
   const unsigned n = e.off[e.nb_total];
@@ -370,7 +370,8 @@ int enqueue_engine_step(tecs_engine* e, float dt) {
   const unsigned chunks = cdiv(len, kScanChunk);
   k_ecount<<<gb, 256, 0, e->stream>>>(e->A, e->Asim, e->ctr, e->table, e->key, e->rank, e->cnt);
   if (chunks > 1) {  // one chunk: its prefix needs no partial sums
-    ECK(cudaMemsetAsync(e->part + chunks, 0, (scan_part_words(len) - chunks) * 4, e->stream));
+    if (chunks > kScanSuper)
+      ECK(cudaMemsetAsync(e->part + chunks, 0, (scan_part_words(len) - chunks) * 4, e->stream));
     k_scan_reduce<<<chunks, kScanThreads, 0, e->stream>>>(e->cnt, len, e->part);
   }
   e->kernels = chunks > 1 ? 7 : 6;

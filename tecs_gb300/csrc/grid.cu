@@ -104,7 +104,7 @@ int grid_rebuild_from_device(tecs_grid* G, const float* pts, unsigned n) {
   const unsigned pw = (unsigned)scan_part_words(len);
   k_count<<<gb, 256, 0, G->stream>>>(G->A, G->ctr, G->g, G->dims, G->key, G->rank, G->cnt, nullptr);
   if (chunks > 1) {
-    GCK(cudaMemsetAsync(G->part + chunks, 0, (size_t)(pw - chunks) * 4, G->stream));
+    if (chunks > kScanSuper) GCK(cudaMemsetAsync(G->part + chunks, 0, (size_t)(pw - chunks) * 4, G->stream));
     k_scan_reduce<<<chunks, kScanThreads, 0, G->stream>>>(G->cnt, len, G->part);
   }
   k_scan_apply<<<chunks, kScanThreads, 0, G->stream>>>(G->cnt, len, G->part, G->off);

@@ -420,7 +420,7 @@ int enqueue_rebuild(tecs_sim* s, int& K, bool run_count) {
     } else if (chunks > 1) {
       // one chunk: its prefix needs no partial sums
       PROF_BEGIN(s);
-      CK(cudaMemsetAsync(s->part + chunks, 0, (pw - chunks) * 4, s->stream));
+      if (chunks > kScanSuper) CK(cudaMemsetAsync(s->part + chunks, 0, (pw - chunks) * 4, s->stream));
       k_scan_reduce<<<chunks, kScanThreads, 0, s->stream>>>(s->cnt, len, s->part);
       PROF_END(s, "k_scan_reduce");
       K += 1;
@@ -538,8 +538,10 @@ int enqueue_pass(tecs_sim* s, PassArgs a, int& K) {
   PROF_BEGIN(s);
   if (!sym && !s->binned && s->d.finder != TECS_FINDER_DELAUNAY)
     fn<<<ceil_div(L ? L : 1, kNaiveThreads / 32 * naive_cells(s)), kNaiveThreads, 0, s->stream>>>(s->g, s->fp, a);
-  else
-    fn<<<ceil_div(L ? L : 1, kPassThreads), kPassThreads, 0, s->stream>>>(s->g, s->fp, a);
+  else {
+    const unsigned threads = !sym && coop_pass(s) ? (s->d.force == 2 ? kCoopThreads<2> : kCoopThreads<1>) : kPassThreads;
+    fn<<<ceil_div(L ? L : 1, threads), threads, 0, s->stream>>>(s->g, s->fp, a);
+  }
   PROF_END(s, a.mode == kStore ? "k_pass_store" : a.mode == kEulerFused ? "k_pass_euler"
               : a.mode == kHeun1Fused ? "k_pass_heun1" : "k_pass_heun2");
   K += 1;
