@@ -1580,6 +1580,23 @@ struct BallBins {
   }
 };
 
+constexpr unsigned kNoRow = 0xffffffffu;
+
+// The slots of n rows of bins [lo, hi), from the bin offsets.
+template <int N>
+__device__ __forceinline__ void row_slots(const unsigned* __restrict__ off, unsigned* lo, unsigned* hi) {
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    const bool ok = lo[r] != kNoRow;
+    const unsigned b = lo[r], e = hi[r];
+    lo[r] = ok ? __ldg(&off[b]) : 0u;
+    hi[r] = ok ? __ldg(&off[e]) : 0u;
+  }
+}
+
+#define TECS_NO_ROW kNoRow
+#define TECS_LOAD(p) __ldg(p)
+#define TECS_ROW_SLOTS(N, lo, hi) row_slots<N>(off, lo, hi)
 #define TECS_WITNESS (FINDER == 3)
 #define TECS_ANY_WITNESS (FINDER == 3)
 #define TECS_PAIR_G(c) g
@@ -1594,13 +1611,13 @@ struct BallBins {
     if (s_ < a.pair_cap)                                                                      \
       a.pairs[s_] = make_uint2(id_at(a.X, a.Bid, i - (unsigned)lane + (c)), id_at(a.X, a.Bid, (jj))); \
   }
-#define TECS_PASS_BODY(BLK, THREADS)                                                          \
+#define TECS_PASS_BODY                                                                        \
   static_assert(FORCE <= 1 || (FORCE == 2 && D == 3), "spring laws, or the 3-D polarity law"); \
   static_assert(FINDER == 1 || FINDER == 3, "the binned finders");                            \
   constexpr bool POL = FORCE == 2;                                                            \
-  constexpr int TB = (THREADS);                                                               \
+  constexpr int TB = kCoopThreads<FORCE>;                                                     \
   const unsigned n = a.ctr->n;                                                                \
-  const unsigned i = (BLK)*TB + threadIdx.x;                                                  \
+  const unsigned i = blockIdx.x * TB + threadIdx.x;                                           \
   const bool run = i < n;                                                                     \
   const float4* const X = a.X;                                                                \
   const float2* const P = a.P;                                                                \
@@ -1627,20 +1644,351 @@ struct BallBins {
 template <int D, int FORCE, int FINDER = 3>
 static __global__ void __launch_bounds__(kCoopThreads<FORCE>, kCoopBlocks)
     k_pass_gabriel(GridP g, ForceP fp, PassArgs a) {
-  TECS_PASS_BODY(blockIdx.x, kCoopThreads<FORCE>)
+  TECS_PASS_BODY
 #include "pass_gabriel_body.inc"
   TECS_PASS_END
 }
 
-// One block's cells blk * kPassThreads .. (only warp-level synchronisation,
-// so a kernel may run several blocks' cells one after another).
-template <int D, int FORCE, int FINDER = 3>
-__device__ __forceinline__ void pass_gabriel_block(const GridP& g, const ForceP& fp, const PassArgs& a,
-                                                   const unsigned blk) {
-  TECS_PASS_BODY(blk, kPassThreads)
-#include "pass_gabriel_body.inc"
-  TECS_PASS_END
+// ---------------------------------------------------------------------------
+// Euler steps of a small simulation in one launch of one cluster of
+// kSmallCtas blocks (up to kSmallCells = 1536 cells and kSmallBins bins; the
+// binned finders on the geometry of the cooperative pass, no COM fix, no
+// division, no links, no extra fields, built-in laws).
+//
+// What bounds such a step is the chain of dependent memory round trips and
+// barriers, so there are few of either.  Every block reads all cells and
+// sorts them by (bin, id) for itself, in shared memory: a coarse histogram of
+// the bin numbers, its scan, the cells grouped by it, and each cell's place
+// among the few of its group.  The rows' slots come from the
+// sorted keys, so no bin counts, offsets or sorted arrays pass between blocks.
+// Each block then takes its own share of the cells, a warp a cell (with a lane
+// a cell, as in the pass over the grid, the two warps of a share take 24,000
+// cycles a step: nothing else runs beside them).  A block writes its cells' new state once
+// all blocks have read the old one: they arrive at the cluster's barrier after
+// their reads and wait before their writes, a whole pass later.  A second
+// barrier ends a step, and the next one follows in the same launch.
+// The arithmetic is that of the passes over the grid: bit-identical runs.
+// 1000 cells, all-pairs: 25 -> 7.7 us a step (counts, scan, scatter and gather
+// through global memory between four cluster barriers, one launch a step: 21;
+// over the grid: 23).
+// The cluster size is set at launch (16 blocks: past the portable 8, opted
+// into per kernel).
+constexpr int kSmallCtas = 16;
+constexpr unsigned kSmallCells = kSmallCtas * kPassThreads;
+constexpr unsigned kSmallBins = 16384;
+constexpr int kSmallThreads = 1024;
+constexpr unsigned kSmallGroups = 2048;                         // of the coarse histogram, four a thread of the scan
+constexpr unsigned kSmallNear = 64;                             // neighbours of a cell
+constexpr int kSmallPer = (int)((kSmallCells + kSmallThreads - 1) / kSmallThreads);  // cells per thread of the sort
+static_assert(kSmallCells <= 2048 && kSmallGroups / 4 <= kSmallThreads, "cells and slots in 11 bits");
+
+// A block's shared memory beside the pass's own.
+struct SmallScratch {
+  float4 x[kSmallCells + 8];                  // sorted positions, w = bin key (the scan reads up to 4 past the end)
+  float2 p[kSmallCells];
+  unsigned long long group[kSmallCells];      // (bin << 22 | id << 11 | slot) grouped by the histogram
+  unsigned key[kSmallCells], id[kSmallCells]; // sorted
+  __align__(16) unsigned coarse[kSmallGroups + 4];  // start of each group
+  unsigned wsum[kSmallThreads / 32];
+  unsigned off[kSmallBins + 1];               // bin offsets, made only where they are needed
+  uint2 rows[kPassThreads * 9];               // the share's rows of bins: their slots
+  float4 near[kSmallThreads / 32][kSmallNear];
+  Acc acc[kPassThreads];                      // the share's sums
+  unsigned general, list[kPassThreads];       // cells that take the general path
+};
+
+// The arrive half of the cluster's barrier and the wait half.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// The first of the sorted keys not below b: in b's group.
+__device__ __forceinline__ unsigned first_key(const SmallScratch& sm, unsigned shift, unsigned b) {
+  unsigned e = sm.coarse[b >> shift];
+  const unsigned end = sm.coarse[(b >> shift) + 1u];
+  while (e < end && sm.key[e] < b) ++e;
+  return e;
 }
+
+// One cell's sums by one warp: its candidates 32 at a time, a lane each; the
+// in-cutoff ones listed in candidate order; a lane a pair for the witness test
+// and the terms, which every lane then adds in that order.  False: more
+// neighbours than the list holds.
+template <int D, int FINDER, int FORCE>
+__device__ __forceinline__ bool small_cell(const GridP& g, const ForceP& fp, const SmallScratch& sm, unsigned n,
+                                           unsigned i, const uint2* rows, float4* near, bool pol, Acc& acc) {
+  constexpr int kRows = D >= 3 ? 9 : 3;
+  const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  acc = Acc{{0.f, 0.f, 0.f}, {0.f, 0.f}};
+  const float4 h = sm.x[i];
+  const uint2 row = lane < (unsigned)kRows ? rows[lane] : make_uint2(0u, 0u);
+  unsigned end = row.y - row.x;  // of the row in the list of candidates
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= (unsigned)o) end += y;
+  }
+  const unsigned total = __shfl_sync(0xffffffffu, end, kRows - 1);
+  const unsigned base = row.y - end;
+  unsigned cnt = 0u;
+  for (unsigned t0 = 0u; t0 < total; t0 += 32u) {
+    const unsigned t = t0 + lane;
+    unsigned r = 0u;
+#pragma unroll
+    for (int k = 0; k < kRows - 1; ++k) r += t >= __shfl_sync(0xffffffffu, end, k) ? 1u : 0u;
+    const unsigned j = t + __shfl_sync(0xffffffffu, base, (int)r);
+    bool in = false;
+    float4 v = h;
+    if (t < total) {
+      v = sm.x[j];
+      const float e0 = h.x - v.x, e1 = h.y - v.y;
+      float d2 = e0 * e0 + e1 * e1;
+      if (D >= 3) { const float e2 = h.z - v.z; d2 = d2 + e2 * e2; }
+      in = d2 < fp.rc2 && j != i;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    const unsigned at = cnt + (unsigned)__popc(m & below);
+    if (in && at < kSmallNear) near[at] = make_float4(v.x, v.y, v.z, __uint_as_float(j));
+    cnt += (unsigned)__popc(m);
+  }
+  if (cnt > kSmallNear) return false;
+  __syncwarp();
+  PolTrig ti{0.f, 0.f, 0.f, 0.f};
+  float2 pi = make_float2(0.f, 0.f);
+  if (FORCE == 2) {
+    pi = sm.p[i];
+    ti = pol_trig(pi);
+  }
+  for (unsigned q0 = 0u; q0 < cnt; q0 += 32u) {
+    const unsigned q = q0 + lane;
+    const bool act = q < cnt;
+    const float4 vj = near[act ? q : 0u];
+    float disp[3] = {h.x - vj.x, h.y - vj.y, D >= 3 ? h.z - vj.z : 0.f};
+    float d2 = disp[0] * disp[0] + disp[1] * disp[1];
+    if (D >= 3) d2 = d2 + disp[2] * disp[2];
+    bool blocked = !act;
+    if (FINDER == 3 && cnt > 1u) {
+      const float m[3] = {h.x - disp[0] * 0.5f, h.y - disp[1] * 0.5f, D >= 3 ? h.z - disp[2] * 0.5f : 0.f};
+      const float rsq = d2 * fp.gab_factor;
+      unsigned long long in = 0ull;
+      for (unsigned w = 0u; w < cnt; ++w) {
+        const float4 vk = near[w];
+        const float e0 = vk.x - m[0], e1 = vk.y - m[1];
+        float s = e0 * e0 + e1 * e1;
+        if (D >= 3) { const float e2 = vk.z - m[2]; s = s + e2 * e2; }
+        if (s < rsq && w != q) in |= 1ull << w;
+      }
+      if (act && in) {
+        const BallBins<D> range(g, m, sqrtf(rsq));
+        for (; in && !blocked; in &= in - 1ull)
+          blocked = range.holds(g, sm.key[__float_as_uint(near[__ffsll((long long)in) - 1].w)]);
+      }
+    }
+    const float dist = sqrtf(d2);
+    float s[3] = {0.f, 0.f, 0.f}, bv[3] = {0.f, 0.f, 0.f}, bp[2] = {0.f, 0.f}, al[2] = {0.f, 0.f};
+    if (!blocked) {
+      if (FORCE != 0) spring_term<D>(fp, disp, dist, s);
+      if (FORCE == 2) {
+        const float2 pj = sm.p[__float_as_uint(vj.w)];
+        polarity_terms(fp, disp, dist, pi, ti, pj, pol_trig(pj), bv, bp, al);
+      }
+    }
+    if (FORCE == 1 && cnt <= 32u) {
+      // (all witnesses have been read: the terms take the list's places, a
+      // blocked pair's +0 leaving the sum, which is never -0, unchanged; lane d
+      // adds component d)
+      __syncwarp();
+      if (act) near[q] = make_float4(s[0], s[1], s[2], 0.f);
+      __syncwarp();
+      float sum = 0.f;
+      const float* term = reinterpret_cast<const float*>(near) + (lane < 3u ? lane : 0u);
+      for (unsigned k = 0u; k < cnt; ++k) sum = sum + term[4u * k];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) acc.x[d] = __shfl_sync(0xffffffffu, sum, d);
+      __syncwarp();
+      return true;
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, !blocked); m && FORCE != 0; m &= m - 1u) {
+      const int k = __ffs(m) - 1;
+#pragma unroll
+      for (int d = 0; d < D; ++d) acc.x[d] = acc.x[d] + __shfl_sync(0xffffffffu, s[d], k);
+      if (FORCE == 2) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) acc.x[d] = acc.x[d] + __shfl_sync(0xffffffffu, bv[d], k);
+#pragma unroll
+        for (int d = 0; d < 2; ++d) acc.p[d] = acc.p[d] + __shfl_sync(0xffffffffu, bp[d], k);
+#pragma unroll
+        for (int d = 0; d < 2; ++d) acc.p[d] = acc.p[d] + __shfl_sync(0xffffffffu, al[d], k);
+      }
+    }
+  }
+  return true;
+}
+
+template <int D, int FINDER, int FORCE>
+static __global__ void __launch_bounds__(kSmallThreads)
+    k_step_small(GridP g, ForceP fp, PassArgs p1, int steps, const float4* A, const float2* PA, float4* B, float2* PB,
+                 unsigned* Bid, unsigned* off_out) {
+  static_assert(FORCE <= 1 || (FORCE == 2 && D == 3), "spring laws, or the 3-D polarity law");
+  extern __shared__ __align__(16) unsigned char small_smem[];
+  SmallScratch& sm = *reinterpret_cast<SmallScratch*>(small_smem);
+  const unsigned n = p1.ctr->n, tid = threadIdx.x;
+  // the block's share: whole warps of cells, spread over the blocks
+  const unsigned share = ((n + kSmallCtas - 1) / kSmallCtas + 31u) & ~31u;
+  const unsigned i0 = min(n, blockIdx.x * share), i1 = min(n, i0 + share);
+  unsigned shift = 0u;
+  while ((g.nbins >> shift) >= kSmallGroups) ++shift;
+  for (int step = 0; step < steps; ++step) {
+    // 1. every block: all cells, counted into groups of bins
+    for (unsigned k = tid; k <= kSmallGroups; k += kSmallThreads) sm.coarse[k] = 0u;
+    float4 v[kSmallPer];
+    unsigned bin[kSmallPer], at[kSmallPer];
+#pragma unroll
+    for (int k = 0; k < kSmallPer; ++k) {
+      const unsigned c = tid + k * kSmallThreads;
+      if (c < n) v[k] = __ldcg(&A[c]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSmallPer; ++k) {
+      const unsigned c = tid + k * kSmallThreads;
+      if (c < n) {
+        const float q[3] = {v[k].x, v[k].y, v[k].z};
+        int b3[3] = {0, 0, 0};
+        bin_coords_div<D>(g, q, b3);
+        bin[k] = flatten<D>(g, b3);
+        at[k] = atomicAdd(&sm.coarse[bin[k] >> shift], 1u);
+      }
+    }
+    __syncthreads();
+    // 2. exclusive scan of the groups' counts, four a thread
+    {
+      const int lane = tid & 31, warp = tid >> 5;
+      const bool part = 4u * tid < kSmallGroups;
+      uint4 c = make_uint4(0u, 0u, 0u, 0u);
+      if (part) c = *reinterpret_cast<const uint4*>(&sm.coarse[4u * tid]);
+      const unsigned own = (c.x + c.y) + (c.z + c.w);
+      unsigned incl = own;
+      if (part) {  // whole warps
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        if (lane == 31) sm.wsum[warp] = incl;
+      }
+      __syncthreads();
+      if (part) {
+        const unsigned before = __reduce_add_sync(0xffffffffu, lane < warp ? sm.wsum[lane] : 0u) + incl - own;
+        const uint4 e = make_uint4(before, before + c.x, before + c.x + c.y, before + c.x + c.y + c.z);
+        *reinterpret_cast<uint4*>(&sm.coarse[4u * tid]) = e;
+        if (4u * tid + 4u == kSmallGroups) sm.coarse[kSmallGroups] = e.w + c.w;
+      }
+    }
+    __syncthreads();
+    // 3. the cells grouped, 4. each one's place by (bin, id)
+#pragma unroll
+    for (int k = 0; k < kSmallPer; ++k) {
+      const unsigned c = tid + k * kSmallThreads;
+      if (c < n)
+        sm.group[sm.coarse[bin[k] >> shift] + at[k]] =
+            (unsigned long long)bin[k] << 22 | (unsigned long long)id_of(v[k]) << 11 | c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSmallPer; ++k) {
+      const unsigned c = tid + k * kSmallThreads;
+      if (c < n) {
+        const unsigned q = bin[k] >> shift, lo = sm.coarse[q], hi = sm.coarse[q + 1u];
+        const unsigned long long me = (unsigned long long)bin[k] << 22 | (unsigned long long)id_of(v[k]) << 11 | c;
+        unsigned dst = lo;
+        for (unsigned e = lo; e < hi; ++e) dst += sm.group[e] < me ? 1u : 0u;
+        sm.x[dst] = make_float4(v[k].x, v[k].y, v[k].z, __uint_as_float(bin[k]));
+        sm.key[dst] = bin[k];
+        sm.id[dst] = id_of(v[k]);
+        if (PA) sm.p[dst] = __ldcg(&PA[c]);
+      }
+    }
+    __syncthreads();
+    cluster_arrive();  // this block has read the state
+    // the sorted copy, by shares
+    for (unsigned s = i0 + tid; s < i1; s += kSmallThreads) {
+      B[s] = sm.x[s];
+      Bid[s] = sm.id[s];
+      if (PB) PB[s] = sm.p[s];
+    }
+    // 5. the slots of the rows of bins around the share's cells
+    constexpr int kRows = D >= 3 ? 9 : 3;
+    const unsigned cells = i1 - i0;
+    if (tid == 0) sm.general = 0u;
+    for (unsigned q = tid; q < cells * kRows; q += kSmallThreads) {
+      const unsigned r = q % kRows;
+      const float4 v4 = sm.x[i0 + q / kRows];
+      const float q3[3] = {v4.x, v4.y, v4.z};
+      int bc[3] = {0, 0, 0};
+      if (FINDER == 1) bin_coords_mul<D>(g, q3, bc);
+      else bin_coords_div<D>(g, q3, bc);
+      const int cy = bc[1] + (int)(r % 3u) - 1, cz = D >= 3 ? bc[2] + (int)(r / 3u) - 1 : 0;
+      unsigned lo = 0u, hi = 0u;
+      if (cy >= 0 && cy < g.ext[1] && (D < 3 || (cz >= 0 && cz < g.ext[2]))) {
+        int c0[3] = {max(bc[0] - 1, 0), cy, cz}, c1[3] = {min(bc[0] + 1, g.ext[0] - 1), cy, cz};
+        lo = first_key(sm, shift, flatten<D>(g, c0));
+        hi = first_key(sm, shift, flatten<D>(g, c1) + 1u);
+      }
+      sm.rows[q] = make_uint2(lo, hi);
+    }
+    __syncthreads();
+    // 6. the cells' forces, one warp a cell
+    for (unsigned c = tid >> 5; c < cells; c += kSmallThreads / 32) {
+      Acc acc;
+      const bool ok = small_cell<D, FINDER, FORCE>(g, fp, sm, n, i0 + c, sm.rows + c * kRows, sm.near[tid >> 5], PA != nullptr, acc);
+      if ((tid & 31u) == 0u) {
+        if (!ok) sm.list[atomicAdd(&sm.general, 1u)] = c;
+        sm.acc[c] = acc;
+      }
+    }
+    __syncthreads();
+    PassArgs a = p1;
+    a.X = sm.x;
+    a.Bx = sm.x;
+    a.P = PA ? sm.p : nullptr;
+    a.Bp = a.P;
+    a.Bid = sm.id;
+    // the bin offsets, for cells that take the general path or for later steps
+    // that keep this sort
+    if (sm.general || off_out) {
+      for (unsigned b = tid; b <= g.nbins; b += kSmallThreads) {
+        const unsigned e = first_key(sm, shift, b);
+        sm.off[b] = e;
+        if (off_out && blockIdx.x == 0) off_out[b] = e;
+      }
+      __syncthreads();
+      a.off = sm.off;
+      if (tid < sm.general) {
+        const unsigned c = sm.list[tid], i = i0 + c;
+        const float4 v4 = sm.x[i];
+        const float xi[3] = {v4.x, v4.y, v4.z};
+        Acc acc = {{0.f, 0.f, 0.f}, {0.f, 0.f}};
+        cell_general<D, FINDER, FORCE>(g, fp, a, n, i, xi, PA ? sm.p[i] : make_float2(0.f, 0.f), 0u, acc);
+        sm.acc[c] = acc;
+      }
+      __syncthreads();
+    }
+    cluster_wait();  // every block has read the state
+    if (tid < cells) {
+      const unsigned i = i0 + tid;
+      const float4 vi = sm.x[i];
+      const float xi[3] = {vi.x, vi.y, vi.z};
+      float s3[3];
+      cell_commit<D>(g, a, n, i, xi, vi, PA ? sm.p[i] : make_float2(0.f, 0.f), sm.acc[tid], s3);
+    }
+    if (step + 1 < steps) {
+      cluster_arrive();
+      cluster_wait();
+    }
+  }
+}
+#undef TECS_NO_ROW
+#undef TECS_LOAD
+#undef TECS_ROW_SLOTS
 #undef TECS_WITNESS
 #undef TECS_ANY_WITNESS
 #undef TECS_PAIR_G
@@ -1717,108 +2065,6 @@ static __global__ void __launch_bounds__(128) k_pass_sym(GridP g, ForceP fp, Pas
   } else {
     for (unsigned j = 0; j < n; ++j) one(j);
   }
-}
-
-// ---------------------------------------------------------------------------
-// One Euler step of a small simulation in one cluster of kSmallCtas blocks
-// (up to kSmallCells = 1536 cells and kSmallBins bins; the binned finders on
-// the geometry of the cooperative pass, no COM fix, no division, no extra
-// fields, built-in laws): the bin counts (made by the previous step's
-// epilogue, or here), their scan, the scatter, the in-bin id order, then the
-// pass -- what the rebuild kernels and the fused pass do over the grid, for a
-// step whose launches would otherwise each cost more than their work.
-// The phases are separated by cluster barriers (release/acquire at cluster
-// scope); every block scans all the counts into its own shared memory, so the
-// scan needs no barrier of its own; each block runs the cooperative pass
-// (pass_gabriel_block) over blocks of cells blockIdx.x, + kSmallCtas, ...  The
-// arithmetic is that of the passes over the grid, so runs are bit-identical.
-// The cluster size is set at launch (16 blocks: past the portable 8, opted
-// into per kernel).
-constexpr int kSmallCtas = 16;
-// one block of cells per block of the cluster: past that the blocks run
-// their cells' blocks in turn, and the grid path spreads them over more SMs
-constexpr unsigned kSmallCells = kSmallCtas * kPassThreads;
-constexpr unsigned kSmallBins = 16384;
-constexpr size_t kSmallSmem = (kSmallBins + 1) * sizeof(unsigned);
-
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-template <int D, int FINDER, int FORCE>
-static __global__ void __launch_bounds__(kPassThreads)
-    k_step_small(GridP g, ForceP fp, PassArgs p1, int run_count, const float4* A, const float2* PA, float4* B,
-                 float2* PB, unsigned* Bid, unsigned* off, unsigned* src, unsigned part_words) {
-  extern __shared__ unsigned offs[];  // the exclusive scan of the counts, nbins + 1 words
-  __shared__ unsigned wsum[kPassThreads / 32];
-  const unsigned n = p1.ctr->n, t = threadIdx.x;
-  const unsigned g0 = blockIdx.x * kPassThreads + t, gs = kSmallCtas * kPassThreads;
-  const int lane = t & 31, warp = t >> 5;
-  const unsigned len = g.nbins + 1;
-  // 1. bin counts of A (the previous step's epilogue made them unless run_count)
-  if (run_count) {
-    for (unsigned c = g0; c < n; c += gs) {
-      const float4 v = A[c];
-      const float q[3] = {v.x, v.y, v.z};
-      int b3[3] = {0, 0, 0};
-      bin_coords_div<D>(g, q, b3);
-      const unsigned b = flatten<D>(g, b3);
-      p1.key[c] = b;
-      p1.rank[c] = atomicAdd(&p1.cnt[b], 1u);
-    }
-    cluster_barrier();
-  }
-  // 2. every block: the exclusive scan of all the counts (offs[nbins] = n);
-  // block 0 also writes it to off for the pass; then the scatter of the
-  // block's own cells
-  {
-    const unsigned per = (len + kPassThreads - 1) / kPassThreads;
-    const unsigned b0 = min(len, t * per), b1 = min(len, b0 + per);
-    unsigned sum = 0;
-    for (unsigned b = b0; b < b1; ++b) sum += p1.cnt[b];
-    unsigned incl = sum;
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (lane == 31) wsum[warp] = incl;
-    __syncthreads();
-    unsigned before = 0;
-    for (int w = 0; w < warp; ++w) before += wsum[w];
-    unsigned run = before + incl - sum;
-    for (unsigned b = b0; b < b1; ++b) {
-      const unsigned c = p1.cnt[b];
-      offs[b] = run;
-      if (blockIdx.x == 0) off[b] = run;
-      run += c;
-    }
-  }
-  __syncthreads();
-  for (unsigned c = g0; c < n; c += gs) src[offs[p1.key[c]] + p1.rank[c]] = c;
-  cluster_barrier();
-  // 3. the counts cleared for the next step's epilogue (and chunk totals that
-  // the counting formed on a sparse grid), each bin in ascending id
-  // (k_order_gather)
-  for (unsigned b = g0; b < len; b += gs) p1.cnt[b] = 0u;
-  for (unsigned w = g0; w < part_words; w += gs) p1.part[w] = 0u;
-  for (unsigned u = g0; u < n; u += gs) {
-    const unsigned c = src[u], b = p1.key[c], lo = offs[b], hi = offs[b + 1];
-    const float4 v = A[c];
-    unsigned dst = u;
-    if (hi - lo > 1u) {
-      const unsigned me = id_of(v);
-      unsigned r = 0;
-      for (unsigned k = lo; k < hi; ++k) r += id_of(A[src[k]]) < me ? 1u : 0u;
-      dst = lo + r;
-    }
-    B[dst] = make_float4(v.x, v.y, v.z, __uint_as_float(b));
-    Bid[dst] = id_of(v);
-    if (PB) PB[dst] = PA[c];
-  }
-  cluster_barrier();
-  // 4. the Euler pass
-  for (unsigned blk = blockIdx.x; blk * kPassThreads < n; blk += kSmallCtas)
-    pass_gabriel_block<D, FORCE, FINDER>(g, fp, p1, blk);
 }
 
 // Plain COM reduction over a delta buffer (used after the symmetric pass).

@@ -148,6 +148,9 @@ static __global__ void k_eorder_gather(const unsigned* __restrict__ off, unsigne
 // POL: some resident simulation carries polarity; spring-only engines use the
 // instance without the polarity law's terms.
 // TB: threads per block (64, 96 or 128; the autotuner's choice).
+#define TECS_NO_ROW kNoRow
+#define TECS_LOAD(p) __ldg(p)
+#define TECS_ROW_SLOTS(N, lo, hi) row_slots<N>(off, lo, hi)
 #define TECS_WITNESS gab
 #define TECS_ANY_WITNESS true
 #define TECS_PAIR_G(c) e.table[hsim[warp * 32 + (c)]].g
@@ -246,6 +249,9 @@ static __global__ void __launch_bounds__(TB, (POL ? 672 : 896) / TB) k_epass(Eng
   e.PA[i] = pn;
   e.Asim[i] = sim;
 }
+#undef TECS_NO_ROW
+#undef TECS_LOAD
+#undef TECS_ROW_SLOTS
 #undef TECS_WITNESS
 #undef TECS_ANY_WITNESS
 #undef TECS_PAIR_G

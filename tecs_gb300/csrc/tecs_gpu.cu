@@ -225,6 +225,7 @@ struct tecs_sim {
   int last_kernels = 0;
   // the next rebuild's bin count is done by the state-writing kernel
   bool fuse_count = false;
+  bool counted = false;  // ... and has been, for the present state (small steps make none)
   bool small_ok = true;  // small steps may take k_step_small (TECS_NO_SMALL_STEP=1: never)
   // sparse grids (bins > 4 x capacity): the counting also forms the scan's
   // chunk totals, and the rebuild needs no reduction pass over the bins
@@ -561,7 +562,7 @@ bool small_step_ok(const tecs_sim* s) {
 }
 
 using SmallFn = void (*)(GridP, ForceP, PassArgs, int, const float4*, const float2*, float4*, float2*, unsigned*,
-                         unsigned*, unsigned*, unsigned);
+                         unsigned*);
 
 SmallFn small_fn_of(const tecs_sim* s) {
   const int D = s->d.dims, F = s->d.finder, FO = s->d.force;
@@ -580,13 +581,12 @@ SmallFn small_fn_of(const tecs_sim* s) {
 
 // Every instantiation of the kernel (the force may change after creation,
 // tecs_sim_set_force), allowed a cluster of kSmallCtas blocks (past the
-// portable 8) and shared memory for the scan of up to kSmallBins + 1 counts
-// past the default 48 KB; set once per device, at the first creation, outside
+// portable 8) and its shared memory past the default 48 KB; set once per device, at the first creation, outside
 // any stream capture.  False if such a cluster cannot be placed on the GPU
 // (steps then run over the grid).
 bool small_prepare_one(SmallFn fn) {
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem) != cudaSuccess) {
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallScratch)) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -597,8 +597,8 @@ bool small_prepare_one(SmallFn fn) {
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(kSmallCtas);
-  cfg.blockDim = dim3(kPassThreads);
-  cfg.dynamicSmemBytes = kSmallSmem;
+  cfg.blockDim = dim3(kSmallThreads);
+  cfg.dynamicSmemBytes = sizeof(SmallScratch);
   cfg.attrs = at;
   cfg.numAttrs = 1;
   int clusters = 0;
@@ -610,6 +610,7 @@ bool small_prepare_one(SmallFn fn) {
 }
 
 constexpr int kMaxDevices = 64;
+constexpr int kSmallSteps = 256;  // of a small simulation in one launch
 
 bool small_prepare(int device) {
   static std::atomic<int> state[kMaxDevices];  // 0 not yet, 1 ready, 2 unavailable
@@ -625,7 +626,13 @@ bool small_prepare(int device) {
   return ok;
 }
 
-int launch_small(tecs_sim* s, SmallFn fn, const PassArgs& p1, bool pol) {
+int launch_small(tecs_sim* s, float dt, double dt64, int steps) {
+  const bool pol = s->d.has_polarity != 0;
+  const SmallFn fn = small_fn_of(s);
+  if (!fn) return fail("unsupported finder/force/dims combination");
+  PassArgs p1 = base_args(s, dt, dt64);
+  p1.mode = kEulerFused;
+  p1.count_next = 0;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -633,14 +640,30 @@ int launch_small(tecs_sim* s, SmallFn fn, const PassArgs& p1, bool pol) {
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(kSmallCtas);
-  cfg.blockDim = dim3(kPassThreads);
-  cfg.dynamicSmemBytes = (s->g.nbins + 1) * sizeof(unsigned);
+  cfg.blockDim = dim3(kSmallThreads);
+  cfg.dynamicSmemBytes = sizeof(SmallScratch);
   cfg.stream = s->stream;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  const unsigned part_words = s->fuse_part ? (unsigned)scan_part_words(s->g.nbins + 1) : 0u;
-  CK(cudaLaunchKernelEx(&cfg, fn, s->g, s->fp, p1, s->fuse_count ? 0 : 1, (const float4*)s->A, (const float2*)(pol ? s->PA : nullptr), s->B,
-                        pol ? s->PB : nullptr, s->Bid, s->off, s->src, part_words));
+  // steps without a rebuild read the bin offsets of this sort
+  unsigned* off_out = s->d.rebuild_every_n > 1 ? s->off : nullptr;
+  CK(cudaLaunchKernelEx(&cfg, fn, s->g, s->fp, p1, steps, (const float4*)s->A, (const float2*)(pol ? s->PA : nullptr),
+                        s->B, pol ? s->PB : nullptr, s->Bid, off_out));
+  return 0;
+}
+
+// The bin counts of A, where steps that did not make them went before
+// (k_step_small).
+int ensure_counted(tecs_sim* s) {
+  if (!s->fuse_count || s->counted) return 0;
+  const unsigned len = s->g.nbins + 1, L = launch_count(s);
+  CK(cudaMemsetAsync(s->cnt, 0, (size_t)len * 4, s->stream));
+  if (s->fuse_part) CK(cudaMemsetAsync(s->part, 0, scan_part_words(len) * 4, s->stream));
+  if (L)
+    k_count<<<ceil_div(L, 256), 256, 0, s->stream>>>(s->A, s->ctr, s->g, s->d.dims, s->key, s->rank, s->cnt,
+                                                     s->fuse_part ? s->part : nullptr);
+  CK(cudaGetLastError());
+  s->counted = true;
   return 0;
 }
 
@@ -669,17 +692,8 @@ int enqueue_step(tecs_sim* s, double dt64, bool rebuild, int& K) {
   PassArgs a = base_args(s, dt, dt64);
   if (rebuild && small_step_ok(s)) {
     // the whole step in one cluster (k_step_small)
-    PassArgs p1 = a;
-    p1.X = s->B;
-    p1.P = pol ? s->PB : nullptr;
-    p1.Bx = s->B;
-    p1.Bp = p1.P;
-    p1.mode = kEulerFused;
-    p1.count_next = s->fuse_count ? 1 : 0;
-    const SmallFn fn = small_fn_of(s);
-    if (!fn) return fail("unsupported finder/force/dims combination");
     PROF_BEGIN(s);
-    if (launch_small(s, fn, p1, pol)) return -1;
+    if (launch_small(s, dt, dt64, 1)) return -1;
     PROF_END(s, "k_step_small");
     K += 1;
     return 0;
@@ -985,13 +999,16 @@ static int upload_common(tecs_sim* s, const float* pos, const float2* pol, unsig
   // the first rebuild expects the bin counts of A, and their chunk totals,
   // to be made already
   const unsigned len = s->g.nbins + 1;
-  if (s->fuse_count) {
+  // (a simulation of small steps needs none)
+  const bool count = s->fuse_count && !small_step_ok(s);
+  s->counted = count;
+  if (count) {
     CK(cudaMemsetAsync(s->cnt, 0, (size_t)len * 4, s->stream));
     if (s->fuse_part) CK(cudaMemsetAsync(s->part, 0, scan_part_words(len) * 4, s->stream));
   }
   k_upload<<<std::max(1u, ceil_div(n, 256)), 256, 0, s->stream>>>(
       pos, s->d.has_polarity ? pol : nullptr, n, s->d.dims, s->A, s->PA, s->ctr, s->g, s->key, s->rank,
-      s->fuse_count ? s->cnt : nullptr, (s->fuse_count && s->fuse_part) ? s->part : nullptr);
+      count ? s->cnt : nullptr, (count && s->fuse_part) ? s->part : nullptr);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(s->stream));
   // the captured step graphs depend on the state only through their grid
@@ -1037,11 +1054,28 @@ int tecs_sim_step(tecs_sim* s, double dt, int n_steps) {
   if (!s) return fail("null simulation");
   if (n_steps < 0) return fail("negative step count");
   CK(cudaSetDevice(s->d.device));
+  if (small_step_ok(s) && s->d.rebuild_every_n <= 1 && !s->profiling) {
+    // every step sorts the cells anew: many steps a launch (at most
+    // kSmallSteps, about two milliseconds)
+    for (int done = 0; done < n_steps; done += kSmallSteps)
+      if (launch_small(s, (float)dt, dt, std::min(kSmallSteps, n_steps - done))) return -1;
+    if (n_steps > 0) {
+      s->step_count = 1;
+      s->last_kernels = 1;
+      s->sorted = true;
+      s->counted = false;
+    }
+    return 0;
+  }
   for (int it = 0; it < n_steps; ++it) {
     // binned_gabriel.hpp:83-89: rebuild when step_count == 0 || step_count >= rebuild_every_n;
     // division resets the counter every step (set_agent_count, :61-64)
     const bool rebuild = s->step_count == 0 || s->step_count >= s->d.rebuild_every_n;
     const int gk = rebuild ? 0 : 1;
+    // a rebuild over the grid starts from the counts of the present state, and
+    // the step's last kernel makes those of the next
+    if (rebuild && small_step_ok(s)) s->counted = false;
+    else if (rebuild && ensure_counted(s)) return -1;
     if (rebuild) s->step_count = 0;
     s->step_count++;
     if (s->d.division_probability > 0.0) s->step_count = 0;
@@ -1146,7 +1180,7 @@ int tecs_sim_evaluate(tecs_sim* s, float* dpos, float* dpol, uint32_t* pairs, si
   if (tecs_sim_count(s, &n)) return -1;
   const bool pol = s->d.has_polarity != 0;
   int K = 0;
-  if (enqueue_rebuild(s, K, !s->fuse_count)) return -1;
+  if (ensure_counted(s) || enqueue_rebuild(s, K, !s->fuse_count)) return -1;
   uint2* dpairs = nullptr;
   if (pairs && pair_cap) CK(cudaMalloc(&dpairs, pair_cap * sizeof(uint2)));
   CK(cudaMemsetAsync(&s->ctr->pair_count, 0, 8, s->stream));

@@ -83,3 +83,46 @@ def test_engine_runs_are_the_plain_ones(finder):
         plain.take_step(0.01, 3)
         np.testing.assert_array_equal(eng.download(slot)[0], plain.get_state()[0])
     eng.close()
+
+
+@pytest.mark.parametrize("n,density", [(1, 1.0), (2, 1.0), (31, 1.0), (700, 0.1), (1000, 1.0), (1000, 9.0), (1200, 60.0),
+                                       (1535, 1.0), (1536, 2.4)])
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("finder", list(FINDERS))
+def test_small_steps(n, density, dims, finder):
+    # one launch, a warp a cell: few and many cells a block, more candidates
+    # than lanes, more neighbours than the list holds (the general path)
+    x = cells(n, density, 11, dims) if n > 2 else wl.ball(n, 11)[:, :dims].copy()
+    s, o = both(x, finder, integrator="euler")
+    s.take_step(0.01, 3)
+    o.step(0.01, 3)
+    bins = np.prod([np.ceil(s.desc.max_bounds[k] - s.desc.min_bounds[k]) for k in range(dims)])
+    assert (s.kernels_per_step() == 1) == (bins <= 16384)  # a sparse grid's steps go over the grid
+    np.testing.assert_array_equal(s.get_state()[0], o.get_state()[0])
+    check(s, o, steps=2)
+
+
+def test_small_steps_in_several_launches_and_then_over_the_grid():
+    # 300 steps are two launches; links then take the steps to the grid, whose
+    # rebuild needs the bin counts that small steps do not make
+    x = cells(600, 1.0, 12)
+    s, o = both(x, "binned_gabriel", integrator="euler")
+    s.take_step(0.01, 300)
+    o.step(0.01, 300)
+    np.testing.assert_array_equal(s.get_state()[0], o.get_state()[0])
+    plain = tg.Simulation(tg.Settings(agent_count=600, capacity=601,  # (another capacity: another simulation)
+                                      pair_finder_settings=tg.PairFinderSettings(
+                                          min_bounds=tuple(s.desc.min_bounds), max_bounds=tuple(s.desc.max_bounds))),
+                          integrator="euler")
+    plain.set_state(s.get_state()[0])
+    links = np.array([[0, 5], [7, 300], [599, 1]], np.uint32)
+    for sim in (s, plain):
+        sim.set_links(links, 0.3)
+        sim.take_step(0.01, 2)
+    assert s.kernels_per_step() > 1
+    np.testing.assert_array_equal(s.get_state()[0], plain.get_state()[0])
+    for sim in (s, plain):
+        sim.set_links(np.zeros((0, 2), np.uint32), 0.0)
+        sim.take_step(0.01, 2)
+    assert s.kernels_per_step() == 1
+    np.testing.assert_array_equal(s.get_state()[0], plain.get_state()[0])
