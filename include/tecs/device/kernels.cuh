@@ -82,7 +82,7 @@ struct PassArgs {
   unsigned* cnt;
   unsigned* part;       // scan chunk totals formed while counting (count_bin), or null
   // naive Delaunay: how many times each directed pair is applied, row i at i * capacity
-  const unsigned short* dmult;
+  const unsigned* dmult;
   // Delaunay (any capacity): cell i's partners and their applications,
   // dl_row[i * kDlRow + t] = (j, reps) for t < dl_len[i], ascending j
   const uint2* dl_row;
@@ -603,10 +603,12 @@ __device__ __forceinline__ bool delaunay_inside(const float4& pm, const float* c
 }
 
 constexpr int kDelaunayThreads = 256;
-constexpr unsigned kDelaunayMaxCells = 4096;  // the pair-count table is capacity^2 x 2 bytes
-// Blocks per cell: block (i, s) takes the in-cutoff pairs number s, s +
-// kDelaunaySplit, ... of cell i.
-constexpr unsigned kDelaunaySplit = 4;
+constexpr unsigned kDelaunayMaxCells = 4096;  // the pair-count table is capacity^2 x 4 bytes
+// Blocks per cell: the third points are dealt to their warps in turn, so that
+// a cell with many pairs takes no longer than its share of the GPU (with the
+// pairs dealt to four blocks the SMs waited 36 % of 2.0 ms for the last ones,
+// 400 cells in 3-D).
+constexpr unsigned kDelaunaySplit = 16;
 constexpr unsigned kDelaunayNear = 64;  // points near i that each simplex is tested against first
 
 // Every simplex is an existence test over all points: one point inside rejects
@@ -617,14 +619,14 @@ constexpr unsigned kDelaunayNear = 64;  // points near i that each simplex is te
 // and its lanes the fourth points l > k; the first accepted l ends k.  2-D:
 // the lanes take the third points.
 // What bounds it: instruction issue (the spheres' arithmetic).  One thread per
-// third point that walks every l and every m in index order (the form before)
-// takes 400-660 ms on 400 cells in 3-D.
+// third point that walks every l and every m in index order takes 400-660 ms
+// on 400 cells in 3-D, this form 1.4 ms.
 template <int D>
 static __global__ void __launch_bounds__(kDelaunayThreads)
 k_delaunay_mult(const float4* __restrict__ X, const Counters* __restrict__ ctr, float rc2, unsigned stride,
-                unsigned short* __restrict__ mult) {
+                unsigned* __restrict__ mult) {  // (cleared before)
   __shared__ float4 near[kDelaunayNear];  // w: the point's index
-  __shared__ unsigned nnear, cnt;
+  __shared__ unsigned nnear;
   const unsigned n = ctr->n;
   const unsigned i = blockIdx.x;
   if (i >= n) return;
@@ -651,7 +653,22 @@ k_delaunay_mult(const float4* __restrict__ X, const Counters* __restrict__ ctr, 
     __syncthreads();
   }
   const unsigned nn = min(nnear, kDelaunayNear);
-  unsigned pair = 0;  // in-cutoff pairs met so far, the same in every thread
+  // nearest first: most spheres fall to the first few
+  {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    unsigned rank = 0u;
+    if (t < nn) {
+      v = near[t];
+      const float d = sq_dist<D>(v, ci);
+      for (unsigned m = 0; m < nn; ++m) {
+        const float e = sq_dist<D>(near[m], ci);
+        rank += (e < d || (e == d && m < t)) ? 1u : 0u;
+      }
+    }
+    __syncthreads();
+    if (t < nn) near[rank] = v;
+    __syncthreads();
+  }
   for (unsigned j0 = 0; j0 < n; j0 += 32u) {
     const unsigned jl = j0 + lane;
     bool in = false;
@@ -662,17 +679,13 @@ k_delaunay_mult(const float4* __restrict__ X, const Counters* __restrict__ ctr, 
       if (D >= 3) { const float e2 = pi.z - v.z; d2 = d2 + e2 * e2; }
       in = !(d2 >= rc2);
     }
-    for (unsigned bits = __ballot_sync(0xffffffffu, in); bits; bits &= bits - 1u, ++pair) {
-      if (pair % kDelaunaySplit != blockIdx.y) continue;
+    for (unsigned bits = __ballot_sync(0xffffffffu, in); bits; bits &= bits - 1u) {
       const unsigned j = j0 + (unsigned)__ffs(bits) - 1u;
       const float4 pj = __ldg(&X[j]);
       const float lj = sq_len<D>(pj);
-      __syncthreads();  // the previous pair's count has been read
-      if (t == 0) cnt = 0u;
-      __syncthreads();
       unsigned local = 0;
       const unsigned items = D == 3 ? n : (n + 31u) / 32u;
-      for (unsigned q = warp; q < items; q += kDelaunayThreads / 32) {
+      for (unsigned q = blockIdx.y + warp * kDelaunaySplit; q < items; q += kDelaunayThreads / 32 * kDelaunaySplit) {
         if (D == 3 && (q == i || q == j)) continue;
         const float4 pq = D == 3 ? __ldg(&X[q]) : pj;
         const float lq = sq_len<3>(pq);
@@ -714,9 +727,7 @@ k_delaunay_mult(const float4* __restrict__ X, const Counters* __restrict__ ctr, 
           if (D == 3 && accepted) break;
         }
       }
-      if (lane == 0u && local) atomicAdd(&cnt, local);
-      __syncthreads();
-      if (t == 0) mult[(size_t)i * stride + j] = (unsigned short)cnt;
+      if (lane == 0u && local) atomicAdd(&mult[(size_t)i * stride + j], local);
     }
   }
 }
