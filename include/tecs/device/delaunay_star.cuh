@@ -501,6 +501,26 @@ TECS_DL_HD bool in_cutoff(const Grid& g, const Pt& pi, const Pt& pj) {
   return d2 < g.rc2;
 }
 
+// Whether the triangle (i, j, k) is not degenerate and none of the points
+// around i (Scratch::kill) rejects it: the start of tri_pass, for one lane.
+template <class S>
+TECS_DL_HD bool tri_near(const Grid& g, unsigned i, unsigned j, unsigned k, const S& sc) {
+  const Pt pi = g.P[i], pj = g.P[j], pk = g.P[k];
+  const float den = 2.0f * (pi.x * (pj.y - pk.y) + pj.x * (pk.y - pi.y) + pk.x * (pi.y - pj.y));
+  if (fabsf(den) <= FLT_EPSILON) return false;
+  const float li = sqlen2(pi), lj = sqlen2(pj), lk = sqlen2(pk);
+  float c[2];
+  c[0] = (li * (pj.y - pk.y) + lj * (pk.y - pi.y) + lk * (pi.y - pj.y)) / den;
+  c[1] = (li * (pk.x - pj.x) + lj * (pi.x - pk.x) + lk * (pj.x - pi.x)) / den;
+  const float e0 = pi.x - c[0], e1 = pi.y - c[1];
+  const float r2 = e0 * e0 + e1 * e1;
+  for (int q = 0; q < sc.n_kill; ++q) {
+    const float f0 = sc.kill[q].x - c[0], f1 = sc.kill[q].y - c[1];
+    if (f0 * f0 + f1 * f1 <= r2 && sc.kill_id[q] != j && sc.kill_id[q] != k) return false;
+  }
+  return true;
+}
+
 // naive_delaunay.hpp:62-99: triangle (i, j, k) accepted
 template <class W, class S>
 TECS_DL_CALL bool tri_pass(const W& w, const Grid& g, unsigned i, unsigned j, unsigned k, const S& sc) {
@@ -592,6 +612,22 @@ TECS_DL_CALL Hit shoot(const W& ln, const Grid& g, const double* x0, const doubl
       ball_at(best.s);
       return best;
     }
+    // a hull edge has no point at all on its open side
+    bool some = false;
+    visit_half<D>(ln, g, pi, w, [&](unsigned id, const Pt& p) {
+      for (int e = 0; e < nex; ++e)
+        if (id == ex[e]) return true;
+      double q[3], wp = 0.0, nn = 0.0;
+      load(p, q);
+      for (int d = 0; d < D; ++d) {
+        const double v = q[d] - pi[d];
+        wp += w[d] * v;
+        nn += v * v;
+      }
+      some = wp > 0.0 && !(wp * wp <= 1.0e-18 * nn);
+      return !some;
+    });
+    if (!ln.any(some)) return best;
   }
   // balls of growing s (doubling in 3-D): in 3-D from the distance from x0 to i (the radius of
   // the empty ball that the search starts from), at least a twentieth of a
@@ -1140,7 +1176,18 @@ TECS_DL_HD unsigned cell_mult(const W& ln, const Grid& g, unsigned i, unsigned* 
       for (int a = 0; a < nn; ++a) {
         const unsigned j = near[a];
         if (!in_cutoff<2>(g, Pi, g.P[j])) continue;
+        // a warp's lanes first put the k to the points around the cell, 32 at a
+        // time: few triangles are left for the test over the grid
+        unsigned left = 0u;
         for (int b = 0; b < nn; ++b) {
+          if (W::width > 1) {
+            const int b0 = b & ~(int)(W::width - 1);
+            if (b == b0) {
+              const int mine = b0 + (int)ln.lane();
+              left = ln.ballot(mine < nn && near[mine] != j && tri_near(g, i, j, near[mine], sc));
+            }
+            if (!(left >> (b - b0) & 1u)) continue;
+          }
           const unsigned k = near[b];
           if (k == j) continue;
           const bool have = find_first(ln, np, [&](int p) { return pairs[p].j == j && pairs[p].k == k; }) >= 0;
