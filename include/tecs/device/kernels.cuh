@@ -1992,6 +1992,7 @@ static __global__ void __launch_bounds__(kSmallThreads)
       cell_commit<D>(g, a, n, i, xi, vi, PA ? sm.p[i] : make_float2(0.f, 0.f), sm.acc[tid], s3);
     }
     if (step + 1 < steps) {
+      __syncwarp();
       cluster_arrive();
       cluster_wait();
     }
