@@ -418,6 +418,8 @@ def run_gb300(args):
     torch.cuda.synchronize()
     value = cell_steps_all / total_s
     kpl = sim.kernels_per_step()
+    # small Euler steps (k_step_small): one launch takes up to 256 of a call's steps
+    launches = -(-chunk // 256) if set(kern) == {"k_step_small"} else kpl * chunk
 
     # End to end through the C ABI with host buffers: every step uploads the
     # state from pinned host memory, steps, and downloads the new state.
@@ -496,10 +498,11 @@ def run_gb300(args):
     pass_launch_s = share * timed_step_s / max(launches_per_step, 1e-9)
     bytes_per_launch = pass_bytes / max(pass_launches, 1)
     achieved = bytes_per_launch * (n_avg / n_prof) / pass_launch_s / 1e9 if pass_launch_s else float("nan")
-    tpc = traffic_per_pass(args.workload)
+    # (the "pass_" figures are those of the pass before its warps shared the cells' work)
+    tpc = pass_profile(args.workload, "dram_bytes_per_cell") or traffic_per_pass(args.workload)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                 "traffic": (tpc * n_avg if tpc else None),
-                "kernel": ("one-launch Euler step (k_step_small: bin sort + pair finding + force + integrator)"
+                "kernel": ("Euler steps in one launch (k_step_small: bin sort + pair finding + force + integrator)"
                            if "k_step_small" in kern else
                            "force pass (k_pass_*: pair finding + force + fused integrator epilogue)"),
                 "bytes_per_launch": bytes_per_launch * n_avg / n_prof,
@@ -512,7 +515,7 @@ def run_gb300(args):
     pass_launches_timed = launches_per_step * len(step_ms) * chunk
     # The pass is bound by instruction issue, not HBM: warp instructions per launch (ncu count per cell x
     # cells) over the live launch time, against SMs x 4 schedulers x the sampled SM clock.
-    ipc = pass_profile(args.workload, "pass_warp_inst_per_cell")
+    ipc = pass_profile(args.workload, "warp_inst_per_cell")
     issue_roofline = None
     if ipc and pass_s:
         sms = torch.cuda.get_device_properties(local).multi_processor_count
@@ -550,7 +553,7 @@ def run_gb300(args):
         "issue_roofline": issue_roofline,
         "cpu_baseline": cpu,
         "e2e": e2e,
-        "gpu_launches": kpl * args.steps * chunk,
+        "gpu_launches": launches * args.steps,
         "kernels": kernel_table,
         "clocks": clocks.summary(),
         "ensemble": ensemble,
