@@ -263,11 +263,21 @@ __device__ __forceinline__ int verify_far(const Warp& w, const Grid& g, unsigned
     for (unsigned k = w.lane(); k < ndone; k += 32u) seen = seen || sc.done[k] == key;
     if (__any_sync(0xffffffffu, seen)) continue;
     const unsigned ia = sc.id[q.x], ib = sc.id[q.y], ic = closed ? sc.id[q.z] : i;
-    const float4 va = sc.p[q.x], vb = sc.p[q.y];
-    float nx = va.y * vb.z - va.z * vb.y, ny = va.z * vb.x - va.x * vb.z, nz = va.x * vb.y - va.y * vb.x;
-    if (q.w == 2) { nx = -nx; ny = -ny; nz = -nz; }
-    // twice the rounding of n: 4 u |a| |b|
-    const float nm = 1.0e-6f * sqrtf(4.0f * va.w * vb.w);
+    // An open face's normal is formed in double: a float one of a thin face may
+    // lean so far that the rows of bins it leaves out hold cells on the open side.
+    double nn[3] = {0.0, 0.0, 0.0}, slack = 0.0;
+    if (!closed) {
+      double a[3], b[3];
+      load(g.P[ia], a);
+      load(g.P[ib], b);
+      for (int d = 0; d < 3; ++d) {
+        const double va = a[d] - pi[d], vb = b[d] - pi[d];
+        a[d] = q.w == 2 ? vb : va;
+        b[d] = q.w == 2 ? va : vb;
+      }
+      if (!plane_normal(a, b, nn, slack)) return 2;
+    }
+    const float nx = (float)nn[0], ny = (float)nn[1], nz = (float)nn[2];
     bool hit = false;
     unsigned hid = 0u;
     float deep = 0.0f;
@@ -279,15 +289,6 @@ __device__ __forceinline__ int verify_far(const Warp& w, const Grid& g, unsigned
       if (dbl && closed) {
         tet_centre(g, pi, ia, ib, ic, xd);
         xx = xd[0] * xd[0] + xd[1] * xd[1] + xd[2] * xd[2];
-      } else if (dbl) {
-        double a[3], b[3];
-        load(g.P[ia], a);
-        load(g.P[ib], b);
-        for (int d = 0; d < 3; ++d) { a[d] -= pi[d]; b[d] -= pi[d]; }
-        cross3(a, b, xd);
-        if (q.w == 2)
-          for (int d = 0; d < 3; ++d) xd[d] = -xd[d];
-        xx = sqrt((a[0] * a[0] + a[1] * a[1] + a[2] * a[2]) * (b[0] * b[0] + b[1] * b[1] + b[2] * b[2]));
       }
       auto test = [&](unsigned e, const Pt& p) {
         if (e == i || e == ia || e == ib || e == ic) return true;
@@ -296,7 +297,8 @@ __device__ __forceinline__ int verify_far(const Warp& w, const Grid& g, unsigned
         bool out, in;
         float depth;
         if (!dbl) {
-          const float lim = closed ? kPowerV * h + kPowerX * c.w : nm * sqrtf(2.0f * h);
+          // (of the plane: the rounding of n and of the products, 16 u |v|)
+          const float lim = closed ? kPowerV * h + kPowerX * c.w : 1.0e-6f * sqrtf(2.0f * h);
           const float pw = closed ? h - (c.x * x + c.y * y + c.z * z) : -(nx * x + ny * y + nz * z);
           out = pw > lim;
           in = pw < -lim;
@@ -304,9 +306,10 @@ __device__ __forceinline__ int verify_far(const Warp& w, const Grid& g, unsigned
         } else {
           const double v[3] = {p.x - pi[0], p.y - pi[1], p.z - pi[2]};
           const double vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-          const double dt = v[0] * xd[0] + v[1] * xd[1] + v[2] * xd[2];
+          const double* to = closed ? xd : nn;
+          const double dt = v[0] * to[0] + v[1] * to[1] + v[2] * to[2];
           const double pw = closed ? 0.5 * vv - dt : -dt;
-          const double lim = closed ? 1.0e-11 * (vv + xx) : 1.0e-13 * xx * sqrt(vv);
+          const double lim = closed ? 1.0e-11 * (vv + xx) : 1.0e-13 * slack * sqrt(vv);
           out = pw > lim;
           in = pw < -lim;
           depth = (float)-pw;
@@ -323,7 +326,6 @@ __device__ __forceinline__ int verify_far(const Warp& w, const Grid& g, unsigned
         const double cc[3] = {pi[0] + c.x, pi[1] + c.y, pi[2] + c.z};
         visit_ball<3>(w, g, cc, (double)(sqrtf(c.w) * 1.0001f), test);
       } else {
-        const double nn[3] = {nx, ny, nz};
         visit_half<3>(w, g, pi, nn, test);
       }
       if (!__any_sync(0xffffffffu, doubt)) break;

@@ -460,6 +460,21 @@ TECS_DL_HD bool visit_half(const W& ln, const Grid& g, const double* o, const do
   }, f);
 }
 
+// The unit normal of the plane through a cell and two others, at a and b from
+// it; slack: |a| |b| over the length of a x b, by which the rounding of a x b
+// (a few 2^-53 |a| |b|) turns the normal.  False where a and b are so nearly on
+// one line that a x b in float (off by up to 7 2^-24 |a| |b|) may point
+// elsewhere, and with it the side of the plane that a float search took.
+TECS_DL_HD bool plane_normal(const double* a, const double* b, double* n, double& slack) {
+  const double c[3] = {a[1] * b[2] - a[2] * b[1], a[2] * b[0] - a[0] * b[2], a[0] * b[1] - a[1] * b[0]};
+  const double len = sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]);
+  const double ab = sqrt((a[0] * a[0] + a[1] * a[1] + a[2] * a[2]) * (b[0] * b[0] + b[1] * b[1] + b[2] * b[2]));
+  if (!(len > 1.0e-5 * ab)) return false;
+  for (int d = 0; d < 3; ++d) n[d] = c[d] / len;
+  slack = ab / len;
+  return true;
+}
+
 // 2-D: every entry within distance del of the line through o with unit
 // normal nrm (and a few just outside): each row of bins cut to the band.
 template <class W, class F, class R>
