@@ -200,7 +200,7 @@ __device__ __forceinline__ void tet_centre(const Grid& g, const double* pi, unsi
 // lies outside their spheres with certainty.
 template <int LOC>
 __device__ __forceinline__ bool verify_tets(const Warp& w, const Grid& g, unsigned i, LocalScratch<LOC>& sc, unsigned n,
-                                            unsigned m) {
+                                            unsigned m, float rho) {
   double pi[3];
   load(g.P[i], pi);
   bool bad = false;
@@ -213,7 +213,7 @@ __device__ __forceinline__ bool verify_tets(const Warp& w, const Grid& g, unsign
     const float x = (float)xd[0], y = (float)xd[1], z = (float)xd[2];
     const float r2 = x * x + y * y + z * z;
     if (t < m) sc.cen[t] = make_float4(x, y, z, r2);
-    if (closed && !(r2 < 1.0e12f)) bad = true;
+    if (closed && !(r2 < 2.5e11f * rho * rho)) bad = true;
     const float m0 = kPowerX * r2;
     for (unsigned k = 0; k < n; ++k) {
       const float4 v = sc.p[k];
@@ -416,20 +416,16 @@ __device__ __forceinline__ bool cell_local3(const Warp& w, const Grid& g, unsign
           nk += (unsigned)__popc(b);
         }
         __syncwarp();
-        float nearest_gap = -1.0e30f;
+        bool doubt = false;  // a line that may bound the face
         for (unsigned k0 = 0; k0 < nk; k0 += 32u) {
           const bool act = k0 + lane < nk;
           const unsigned k = act ? sc.list[k0 + lane] : J;
           const float4 vk = sc.p[k];
-          const float wx = vj.y * vk.z - vj.z * vk.y, wy = vj.z * vk.x - vj.x * vk.z, wz = vj.x * vk.y - vj.y * vk.x;
-          const float w2 = wx * wx + wy * wy + wz * wz;
-          const float inv = 1.0f / w2;
-          // the circumcentre of (i, j, k) in their plane
-          const float x0 = (vj.w * (vk.y * wz - vk.z * wy) + vk.w * (wy * vj.z - wz * vj.y)) * inv;
-          const float y0 = (vj.w * (vk.z * wx - vk.x * wz) + vk.w * (wz * vj.x - wx * vj.z)) * inv;
-          const float z0 = (vj.w * (vk.x * wy - vk.y * wx) + vk.w * (wx * vj.y - wy * vj.x)) * inv;
+          const FaceLine<float> ln = face_line(vj.x, vj.y, vj.z, vj.w, vk.x, vk.y, vk.z, vk.w);
+          const float wx = ln.wx, wy = ln.wy, wz = ln.wz, w2 = ln.w2, inv = ln.inv, x0 = ln.x, y0 = ln.y, z0 = ln.z;
           const float room = 1.02f * r2max - (x0 * x0 + y0 * y0 + z0 * z0);
-          const bool alive = act && w2 > 0.0f && (wide || room > 0.0f);
+          const bool line = act && w2 > kLineMin;
+          const bool alive = line && (wide || room > 0.0f);
           float hi = !alive ? -1.0f : wide ? 1.0e15f : sqrtf(room * inv), lo = -hi;
           unsigned hl = kNoEnd, ll = kNoEnd;
           for (unsigned l0 = 0; l0 < n;) {
@@ -459,7 +455,18 @@ __device__ __forceinline__ bool cell_local3(const Warp& w, const Grid& g, unsign
             l0 = l1;
           }
           const bool member = alive && lo < hi;
-          if (alive && !member) nearest_gap = fmaxf(nearest_gap, (hi - lo) * sqrtf(w2));
+          if (wide && act && !member) {
+            // certain only where the two cuts cross by more than their rounding,
+            // in float or else in double
+            bool apart = false;
+            if (line && hl != kNoEnd && ll != kNoEnd) {
+              const float4 vh = sc.p[hl], vl = sc.p[ll];
+              const CutError<float> err(ln, vj.w, vk.w);
+              apart = (lo - hi) * err.len > err.of(ln, vh.x, vh.y, vh.z, vh.w, hi) + err.of(ln, vl.x, vl.y, vl.z, vl.w, lo) ||
+                      cuts_cross(g.P[i], g.P[sc.id[J]], g.P[sc.id[k]], g.P[sc.id[hl]], g.P[sc.id[ll]]);
+            }
+            doubt = doubt || !apart;
+          }
           // an end at the largest sphere: its tetrahedron reaches out of the ball
           if (!FAR && __any_sync(0xffffffffu, member && (wide || hl == kNoEnd || ll == kNoEnd))) return false;
           members += (unsigned)__popc(__ballot_sync(0xffffffffu, member));
@@ -490,8 +497,10 @@ __device__ __forceinline__ bool cell_local3(const Warp& w, const Grid& g, unsign
           }
           if (tets > 160u) return false;
         }
-        // no face: certain unless a line was missed by no more than the rounding
-        if (wide && members == 0u && __any_sync(0xffffffffu, nearest_gap > -3.0e-5f)) return false;
+        // No face: certain where every line is.  (Where some lines bound the face
+        // and one was missed, its tetrahedra are met from the other third point
+        // alone, and mix is not zero.)
+        if (wide && members == 0u && __any_sync(0xffffffffu, doubt)) return false;
       }
       if (mix != 0u) return false;
       if (reps) {
@@ -504,7 +513,7 @@ __device__ __forceinline__ bool cell_local3(const Warp& w, const Grid& g, unsign
       }
       if (!FAR && tets > 96u) {
         __syncwarp();
-        if (!verify_tets(w, g, i, sc, n, tets)) return false;
+        if (!verify_tets(w, g, i, sc, n, tets, rho)) return false;
         for (unsigned t = lane; t < tets; t += 32u)
           if (!(4.0f * sc.cen[t].w <= rho * rho * 0.9999f)) big = true;
         __syncwarp();
@@ -513,7 +522,7 @@ __device__ __forceinline__ bool cell_local3(const Warp& w, const Grid& g, unsign
     }
   }
   __syncwarp();
-  if (!verify_tets(w, g, i, sc, n, tets)) return false;
+  if (!verify_tets(w, g, i, sc, n, tets, rho)) return false;
   if (FAR) {
     __syncwarp();
     const int far = verify_far(w, g, i, sc, n, tets, rho, ndone);

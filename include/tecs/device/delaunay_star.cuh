@@ -475,6 +475,85 @@ TECS_DL_HD bool plane_normal(const double* a, const double* b, double* n, double
   return true;
 }
 
+// The local search in space (delaunay_local.cuh): the line in which the planes
+// halfway to two others, at vj and vk from the cell, meet -- x + t w with x its
+// point nearest to the cell.  h: half a squared length.
+template <class T>
+struct FaceLine {
+  T wx, wy, wz, w2, inv, x, y, z;
+};
+
+// Lines with a lesser w^2 are not formed in float: their products may underflow.
+constexpr float kLineMin = 1.0e-28f;
+
+template <class T>
+TECS_DL_HD FaceLine<T> face_line(T jx, T jy, T jz, T jh, T kx, T ky, T kz, T kh) {
+  FaceLine<T> l;
+  l.wx = jy * kz - jz * ky;
+  l.wy = jz * kx - jx * kz;
+  l.wz = jx * ky - jy * kx;
+  l.w2 = l.wx * l.wx + l.wy * l.wy + l.wz * l.wz;
+  l.inv = (T)1 / l.w2;
+  l.x = (jh * (ky * l.wz - kz * l.wy) + kh * (l.wy * jz - l.wz * jy)) * l.inv;
+  l.y = (jh * (kz * l.wx - kx * l.wz) + kh * (l.wz * jx - l.wx * jz)) * l.inv;
+  l.z = (jh * (kx * l.wy - ky * l.wx) + kh * (l.wx * jy - l.wy * jx)) * l.inv;
+  return l;
+}
+
+// How far rounding may move the cut that a point makes on a line, as a length.
+// With u the unit roundoff, S the sine of the angle between vj and vk and Q
+// that of a point's v with the plane across the line, rounding moves
+//   w   by 7 u |vj| |vk|                     (a turn of 7 u / S),
+//   x   by 18 u (|vj| + |vk|) / S^2          (|x| <= (|vj| + |vk|) / 2 S),
+//   T   by u (2.5 |v| + 18 (|vj| + |vk|) / S^2 + 4 |x| + |T| (7 / S + 4)) / Q + 3 u |T|
+// of a cut at T = t |w| from x.  Twice that is allowed for, which covers the
+// second order and the rounding here; it holds in any unit of length.
+TECS_DL_HD float root(float v) { return sqrtf(v); }
+TECS_DL_HD double root(double v) { return sqrt(v); }
+TECS_DL_HD float size(float v) { return fabsf(v); }
+TECS_DL_HD double size(double v) { return fabs(v); }
+
+template <class T>
+struct CutError {
+  T len, turn, near;  // |w|, 1 / S, 20 (|vj| + |vk|) / S^2
+  TECS_DL_HD CutError(const FaceLine<T>& l, T jh, T kh) {
+    len = root(l.w2);
+    turn = (T)2 * root(jh) * root(kh) / len;
+    near = (T)28.3 * (root(jh) + root(kh)) * turn * turn;
+  }
+  TECS_DL_HD T of(const FaceLine<T>& l, T vx, T vy, T vz, T vh, T t) const {
+    constexpr T u2 = sizeof(T) == 4 ? (T)1.3e-7 : (T)2.4e-16;
+    const T v = (T)1.4143 * root(vh);
+    const T q = size(l.wx * vx + l.wy * vy + l.wz * vz);
+    return u2 * ((T)3 * v + near + (T)14 * size(t) * len * turn) * (len * v / q);
+  }
+};
+
+// In double: whether the line of the planes halfway to pj and pk is cut off at
+// t < hi by ph and at t > lo by pl with hi < lo, with certainty.
+template <class P>
+TECS_DL_CALL bool cuts_cross(const P& pi, const P& pj, const P& pk, const P& ph, const P& pl) {
+  double v[4][3], h[4];
+  const P* p[4] = {&pj, &pk, &ph, &pl};
+  for (int q = 0; q < 4; ++q) {
+    v[q][0] = (double)p[q]->x - (double)pi.x;
+    v[q][1] = (double)p[q]->y - (double)pi.y;
+    v[q][2] = (double)p[q]->z - (double)pi.z;
+    h[q] = 0.5 * (v[q][0] * v[q][0] + v[q][1] * v[q][1] + v[q][2] * v[q][2]);
+  }
+  const FaceLine<double> l = face_line(v[0][0], v[0][1], v[0][2], h[0], v[1][0], v[1][1], v[1][2], h[1]);
+  const CutError<double> err(l, h[0], h[1]);
+  double t[2], e[2];
+  for (int q = 0; q < 2; ++q) {
+    const double* c = v[2 + q];
+    const double wl = l.wx * c[0] + l.wy * c[1] + l.wz * c[2];
+    if (!(q ? wl < 0.0 : wl > 0.0)) return false;
+    t[q] = (h[2 + q] - (l.x * c[0] + l.y * c[1] + l.z * c[2])) / wl;
+    e[q] = err.of(l, c[0], c[1], c[2], h[2 + q], t[q]);
+  }
+  return (t[1] - t[0]) * err.len > e[0] + e[1];
+}
+
 // 2-D: every entry within distance del of the line through o with unit
 // normal nrm (and a few just outside): each row of bins cut to the band.
 template <class W, class F, class R>

@@ -5,6 +5,12 @@
 //     open faces of cells with two others nearly on one line, on a grid of the
 //     size of 40,000 cells: prints "<angle> <faces> <refused> <points> <missed>",
 //     missed being points on the open side that the rows looked up leave out.
+//   delaunay_margins_host lines
+//     the lines that may bound the Voronoi faces of a cell among its neighbours,
+//     cut in float as the search does and in double: prints
+//     "<set> <unit of length> <lines without a rest in float> <looked at in double>
+//     <doubtful> <wrong>",
+//     wrong being those called certain of which double leaves something.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -88,7 +94,108 @@ static int normals() {
   return 0;
 }
 
+// Neighbourhoods: random cells, lattices with jitter (near-ties), a cell that
+// is nearly on one line with many pairs of others.
+static std::vector<Pt> cloud(int set, double unit, unsigned seed) {
+  std::mt19937 rng(seed);
+  std::normal_distribution<double> nd(0.0, 1.0);
+  std::uniform_real_distribution<double> u11(-1.0, 1.0);
+  std::vector<Pt> p{Pt{0.f, 0.f, 0.f, 0.f}};
+  auto put = [&](double x, double y, double z) {
+    p.push_back(Pt{(float)(unit * x), (float)(unit * y), (float)(unit * z), 0.f});
+  };
+  if (set == 0) {
+    while (p.size() < 90) put(2.8 * u11(rng), 2.8 * u11(rng), 2.8 * u11(rng));
+  } else if (set <= 3) {
+    const double jitter = set == 1 ? 1e-2 : set == 2 ? 1e-4 : 1e-6;
+    for (int x = -2; x <= 2; ++x)
+      for (int y = -2; y <= 2; ++y)
+        for (int z = -1; z <= 1; ++z)
+          if (x || y || z) put(x + jitter * nd(rng), y + jitter * nd(rng), z + jitter * nd(rng));
+  } else {
+    while (p.size() < 90) {
+      const double t = 2.5 * u11(rng);
+      put(t + 1e-3 * nd(rng), 0.3 * t + 1e-3 * nd(rng), 0.5 + (p.size() % 2) * 1e-4 * nd(rng));
+    }
+  }
+  return p;
+}
+
+// What the other points leave of the line of j and k, in long double
+// (80 or 128 bits: below the rounding of cuts_cross).
+static bool rest(const std::vector<Pt>& p, int j, int k) {
+  using L = long double;
+  const L a[3] = {p[j].x, p[j].y, p[j].z}, b[3] = {p[k].x, p[k].y, p[k].z};
+  L ha = 0, hb = 0, w[3], x[3], w2 = 0, hi = 1e300L, lo = -1e300L;
+  for (int d = 0; d < 3; ++d) {
+    const int e = (d + 1) % 3, f = (d + 2) % 3;
+    w[d] = a[e] * b[f] - a[f] * b[e];
+    ha += a[d] * a[d] / 2;
+    hb += b[d] * b[d] / 2;
+    w2 += w[d] * w[d];
+  }
+  for (int d = 0; d < 3; ++d) {
+    const int e = (d + 1) % 3, f = (d + 2) % 3;
+    x[d] = (ha * (b[e] * w[f] - b[f] * w[e]) + hb * (w[e] * a[f] - w[f] * a[e])) / w2;
+  }
+  for (int l = 1; l < (int)p.size(); ++l) {
+    if (l == j || l == k) continue;
+    const L v[3] = {p[l].x, p[l].y, p[l].z};
+    L h = 0, wl = 0, xl = 0;
+    for (int d = 0; d < 3; ++d) {
+      h += v[d] * v[d] / 2;
+      wl += w[d] * v[d];
+      xl += x[d] * v[d];
+    }
+    const L t = (h - xl) / wl;
+    if (wl > 0 && t < hi) hi = t;
+    if (wl < 0 && t > lo) lo = t;
+  }
+  return lo < hi;
+}
+
+static int lines() {
+  for (int set = 0; set < 5; ++set)
+    for (const double unit : {1.0, 37.0, 1000.0, 1024.0, 1.0 / 8192.0, 1e-4}) {
+      unsigned long long none = 0, again = 0, doubtful = 0, wrong = 0;
+      for (unsigned seed = 1; seed <= 6; ++seed) {
+        const std::vector<Pt> p = cloud(set, unit, seed);
+        const int n = (int)p.size();
+        std::vector<float> h(n);
+        for (int a = 0; a < n; ++a) h[a] = 0.5f * (p[a].x * p[a].x + p[a].y * p[a].y + p[a].z * p[a].z);
+        for (int j = 1; j < n; ++j)
+          for (int k = 1; k < n; ++k) {
+            if (k == j) continue;
+            const FaceLine<float> f = face_line(p[j].x, p[j].y, p[j].z, h[j], p[k].x, p[k].y, p[k].z, h[k]);
+            if (!(f.w2 > kLineMin)) continue;
+            float hi = 1e15f, lo = -1e15f;
+            int hl = -1, ll = -1;
+            for (int l = 1; l < n; ++l) {
+              if (l == j || l == k) continue;
+              const float wl = std::fmaf(f.wz, p[l].z, std::fmaf(f.wy, p[l].y, f.wx * p[l].x));
+              const float t = (h[l] - std::fmaf(f.z, p[l].z, std::fmaf(f.y, p[l].y, f.x * p[l].x))) / wl;
+              if (wl > 0.f && t < hi) { hi = t; hl = l; }
+              if (wl < 0.f && t > lo) { lo = t; ll = l; }
+            }
+            if (lo < hi) continue;
+            ++none;
+            const CutError<float> err(f, h[j], h[k]);
+            const bool close = !(hl >= 0 && ll >= 0 &&
+                                 (lo - hi) * err.len > err.of(f, p[hl].x, p[hl].y, p[hl].z, h[hl], hi) +
+                                                           err.of(f, p[ll].x, p[ll].y, p[ll].z, h[ll], lo));
+            const bool apart = !close || (hl >= 0 && ll >= 0 && cuts_cross(p[0], p[j], p[k], p[hl], p[ll]));
+            again += close ? 1u : 0u;
+            if (!apart) ++doubtful;
+            else if (rest(p, j, k)) ++wrong;
+          }
+      }
+      std::printf("%d %.9g %llu %llu %llu %llu\n", set, unit, none, again, doubtful, wrong);
+    }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   if (argc == 2 && !std::strcmp(argv[1], "normals")) return normals();
+  if (argc == 2 && !std::strcmp(argv[1], "lines")) return lines();
   return 2;
 }

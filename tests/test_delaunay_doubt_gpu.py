@@ -2,11 +2,13 @@
 
 Rows have to be the host walk's (tests/cpp/delaunay_star_host.cpp), pair by
 pair, whichever of the searches takes a cell: hull edges that carry cells
-nearly on one line (faces too thin for a float normal).
+nearly on one line (faces too thin for a float normal), and cells in other
+units of length than about one cell a unit.
 """
 import numpy as np
 import pytest
 
+from tecs_gb300 import workloads as wl
 from test_delaunay_local_gpu import expected, found, host_search  # noqa: F401 (a fixture)
 
 pytestmark = pytest.mark.gpu
@@ -29,3 +31,22 @@ def box_with_edges(jitter):
 def test_thin_hull_faces(host_search, jitter):  # noqa: F811
     x = box_with_edges(jitter)
     assert found(x, 1.0) == expected(host_search, x, 1.0)
+
+
+def scaled(kind, unit):
+    rng = np.random.default_rng(13)
+    if kind == "ball":
+        x = wl.ball(3000, 7)
+    else:
+        x = np.stack(np.meshgrid(*[np.arange(11)] * 3, indexing="ij"), -1).reshape(-1, 3) + rng.normal(0, 1e-3, (1331, 3))
+    return (x * unit).astype(np.float32)
+
+
+@pytest.mark.parametrize("unit", [1e-9, 1e-4, 1e-3, 1e3, 5e3, 1e6])
+@pytest.mark.parametrize("kind", ["ball", "near_lattice"])
+def test_units_of_length(host_search, kind, unit):  # noqa: F811
+    x = scaled(kind, unit)
+    cutoff = float(np.float32(1.3 * unit))
+    rows = found(x, cutoff)
+    assert rows == expected(host_search, x, cutoff)
+    assert len(rows) > 3 * len(x)

@@ -32,3 +32,18 @@ def test_rows_of_an_open_face_hold_its_open_side(margins):
         assert int(missed) == 0, (angle, missed)
         assert int(faces) == 60 and (int(points) > 0 or int(refused) == 60)
         assert int(refused) == 0 or float(angle) < 1e-4
+
+
+def test_a_line_called_without_rest_has_none(margins):
+    # near-ties and lines far from the cell: nothing certain may be wrong in
+    # more bits, in any unit of length; one that is a power of two changes no
+    # verdict (but for lines too short to be formed); among random cells next
+    # to nothing is looked at in double (the set of 1e-6 jitter has exact ties)
+    rows = [(int(s), float(u)) + tuple(map(int, c)) for s, u, *c in margins("lines")]
+    assert len(rows) == 30
+    for s, unit, none, again, doubtful, wrong in rows:
+        assert none > 1000 and wrong == 0, (s, unit, wrong)
+        same = next(r for r in rows if r[0] == s and r[1] == 1.0)
+        if unit == 1024.0 or (unit == 1.0 / 8192.0 and s != 3):
+            assert (none, again, doubtful) == same[2:5]
+        assert s > 0 or (doubtful <= again < 0.01 * none), (s, unit, again, doubtful, none)
