@@ -51,6 +51,21 @@ inline void grid_set_constants(GridP& g) {
   g.div_y = grid_divisor((unsigned)g.ext[1]);
 }
 
+// Whether float resolves the grid's positions and bins well enough for the
+// Gabriel fast path's geometry (kernels.cuh): a witness within 0.95 cutoffs of
+// the cell has to be found in cutoff and in the bins around the cell's own.
+// Up to 2^18 cutoffs from the origin and 2^18 bins a side, rounding moves a
+// midpoint by at most 1/64 of a cutoff and a bin's edges by 1/64 of a bin.
+// (At 2^21, five to eleven positions a cutoff, witnesses are missed.)
+inline bool grid_resolved(const GridP& g, float cutoff) {
+  constexpr float kMost = 262144.0f;
+  for (int d = 0; d < 3; ++d) {
+    const float hi = g.mn[d] + (float)g.ext[d] * g.bin_size;
+    if (!((float)g.ext[d] <= kMost && std::fabs(g.mn[d]) <= kMost * cutoff && std::fabs(hi) <= kMost * cutoff)) return false;
+  }
+  return true;
+}
+
 // Built-in force descriptor plus the pair predicates' constants.
 struct ForceP {
   int force;        // tecs_force

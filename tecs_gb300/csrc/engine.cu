@@ -589,7 +589,7 @@ int tecs_engine_add(tecs_engine* e, const tecs_sim_desc* d, const float* positio
   sl.integrator = d->integrator;
   sl.has_pol = d->has_polarity ? 1 : 0;
   sl.active = 1;
-  sl.gabriel_fast = d->gabriel_coefficient <= 0.9f ? 1 : 0;
+  sl.gabriel_fast = (d->gabriel_coefficient <= 0.9f && grid_resolved(g, d->cutoff)) ? 1 : 0;
   // append the cells after the resident ones (the next sort merges them)
   const unsigned at = e->n_resident;
   if (n) {

@@ -277,11 +277,14 @@ int prof_mark(tecs_sim* s, int which, const char* name) {
 // in the 3^dims bins around its own.
 bool coop_geometry(const tecs_sim* s) { return s->g.R == 1 && s->g.bin_size >= s->d.cutoff; }
 // The built-in binned pass over the grid is the cooperative one
-// (k_pass_gabriel): all-pairs on its geometry, Gabriel also with c <= 0.9.
+// (k_pass_gabriel): all-pairs on its geometry, Gabriel also with c <= 0.9 where
+// float resolves the grid (elsewhere the general path looks into every bin of a
+// pair's ball).
 bool coop_pass(const tecs_sim* s) {
   const bool geom = coop_geometry(s);
   if (s->d.finder == TECS_FINDER_BINNED_ALL_PAIRS) return geom;
-  return s->d.finder == TECS_FINDER_BINNED_GABRIEL && geom && s->d.gabriel_coefficient <= 0.9f;
+  return s->d.finder == TECS_FINDER_BINNED_GABRIEL && geom && s->d.gabriel_coefficient <= 0.9f &&
+         grid_resolved(s->g, s->d.cutoff);
 }
 
 // The naive finders' pass: cells per warp.  One cell a warp fills the GPU up
@@ -294,8 +297,7 @@ unsigned naive_cells(const tecs_sim* s) {
 
 PassFn pass_fn(const tecs_sim* s, bool sym) {
   const int D = s->d.dims, F = s->d.finder, FO = s->d.force;
-  const bool coop_geom = coop_geometry(s);
-  const bool coop = coop_geom && s->d.gabriel_coefficient <= 0.9f;
+  const bool coop = coop_pass(s);
 #define PICK(DD, FF)                                                            \
   if (D == DD && F == FF) {                                                     \
     if (sym) {                                                                  \
@@ -306,9 +308,9 @@ PassFn pass_fn(const tecs_sim* s, bool sym) {
       if (FF == 3 && coop && FO == 0) return k_pass_gabriel<DD, 0>;             \
       if (FF == 3 && coop && FO == 1) return k_pass_gabriel<DD, 1>;             \
       if (FF == 3 && coop && FO == 2 && DD == 3) return k_pass_gabriel<3, 2>;   \
-      if (FF == 1 && coop_geom && FO == 0) return k_pass_gabriel<DD, 0, 1>;     \
-      if (FF == 1 && coop_geom && FO == 1) return k_pass_gabriel<DD, 1, 1>;     \
-      if (FF == 1 && coop_geom && FO == 2 && DD == 3) return k_pass_gabriel<3, 2, 1>; \
+      if (FF == 1 && coop && FO == 0) return k_pass_gabriel<DD, 0, 1>;     \
+      if (FF == 1 && coop && FO == 1) return k_pass_gabriel<DD, 1, 1>;     \
+      if (FF == 1 && coop && FO == 2 && DD == 3) return k_pass_gabriel<3, 2, 1>; \
       if (FO == 0) return k_pass<DD, FF, 0>;                                    \
       if (FO == 1) return k_pass<DD, FF, 1>;                                    \
       if (DD == 3) return k_pass<DD, FF, 2>;                                    \
