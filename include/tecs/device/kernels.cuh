@@ -1695,17 +1695,16 @@ static_assert(kSmallCells <= 2048 && kSmallGroups / 4 <= kSmallThreads, "cells a
 
 // A block's shared memory beside the pass's own.
 struct SmallScratch {
-  float4 x[kSmallCells + 8];                  // sorted positions, w = bin key (the scan reads up to 4 past the end)
+  float4 x[kSmallCells];                      // sorted positions, w = bin key
   float2 p[kSmallCells];
   unsigned long long group[kSmallCells];      // (bin << 22 | id << 11 | slot) grouped by the histogram
   unsigned key[kSmallCells], id[kSmallCells]; // sorted
   __align__(16) unsigned coarse[kSmallGroups + 4];  // start of each group
   unsigned wsum[kSmallThreads / 32];
-  unsigned off[kSmallBins + 1];               // bin offsets, made only where they are needed
   uint2 rows[kPassThreads * 9];               // the share's rows of bins: their slots
   float4 near[kSmallThreads / 32][kSmallNear];
   Acc acc[kPassThreads];                      // the share's sums
-  unsigned general, list[kPassThreads];       // cells that take the general path
+  unsigned crowded, list[kPassThreads];       // cells of more neighbours than a list holds
 };
 
 // The arrive half of the cluster's barrier and the wait half.
@@ -1720,26 +1719,129 @@ __device__ __forceinline__ unsigned first_key(const SmallScratch& sm, unsigned s
   return e;
 }
 
-// One cell's sums by one warp: its candidates 32 at a time, a lane each; the
-// in-cutoff ones listed in candidate order; a lane a pair for the witness test
-// and the terms, which every lane then adds in that order.  False: more
-// neighbours than the list holds.
-template <int D, int FINDER, int FORCE>
-__device__ __forceinline__ bool small_cell(const GridP& g, const ForceP& fp, const SmallScratch& sm, unsigned n,
-                                           unsigned i, const uint2* rows, float4* near, bool pol, Acc& acc) {
-  constexpr int kRows = D >= 3 ? 9 : 3;
-  const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-  acc = Acc{{0.f, 0.f, 0.f}, {0.f, 0.f}};
-  const float4 h = sm.x[i];
-  const uint2 row = lane < (unsigned)kRows ? rows[lane] : make_uint2(0u, 0u);
-  unsigned end = row.y - row.x;  // of the row in the list of candidates
+// A cell's rows as one list of candidates: lane r's row is the places up to
+// end, at slots base further on.
+__device__ __forceinline__ void small_rows(const uint2* rows, int n, unsigned& end, unsigned& base) {
+  const unsigned lane = threadIdx.x & 31u;
+  const uint2 row = lane < (unsigned)n ? rows[lane] : make_uint2(0u, 0u);
+  end = row.y - row.x;
 #pragma unroll
   for (int o = 1; o < 16; o <<= 1) {
     const unsigned y = __shfl_up_sync(0xffffffffu, end, o);
     if (lane >= (unsigned)o) end += y;
   }
+  base = row.y - end;
+}
+
+// A cell of more neighbours than the list holds, by one warp: a lane a
+// candidate, 32 at a time; a pair's witnesses are looked for among all the
+// candidates (row by row, each read by all lanes at once), and the terms added in
+// candidate order.
+// What bounds it: instruction issue, (candidates / 32) x candidates x about 14.
+// A thread a cell over the general path (each pair's witnesses one after
+// another, three warps a block) takes 20.5 ms a step for 1,500 cells in a ball
+// of radius 1.5, where this takes 1.
+template <int D, int FINDER, int FORCE>
+__device__ __forceinline__ void small_cell_crowded(const GridP& g, const ForceP& fp, const SmallScratch& sm, unsigned i,
+                                                   const uint2* rows, float4* near, Acc& acc) {
+  constexpr int kRows = D >= 3 ? 9 : 3;
+  const unsigned lane = threadIdx.x & 31u;
+  acc = Acc{{0.f, 0.f, 0.f}, {0.f, 0.f}};
+  unsigned end, base;
+  small_rows(rows, kRows, end, base);
   const unsigned total = __shfl_sync(0xffffffffu, end, kRows - 1);
-  const unsigned base = row.y - end;
+  const float4 h = sm.x[i];
+  PolTrig ti{0.f, 0.f, 0.f, 0.f};
+  float2 pi = make_float2(0.f, 0.f);
+  if (FORCE == 2) {
+    pi = sm.p[i];
+    ti = pol_trig(pi);
+  }
+  float sum = 0.f;  // of component `lane`
+  for (unsigned t0 = 0u; t0 < total; t0 += 32u) {
+    const unsigned t = t0 + lane;
+    unsigned r = 0u;
+#pragma unroll
+    for (int k = 0; k < kRows - 1; ++k) r += t >= __shfl_sync(0xffffffffu, end, k) ? 1u : 0u;
+    const unsigned j = t + __shfl_sync(0xffffffffu, base, (int)r);
+    const float4 v = t < total ? sm.x[j] : h;
+    float disp[3] = {h.x - v.x, h.y - v.y, D >= 3 ? h.z - v.z : 0.f};
+    float d2 = disp[0] * disp[0] + disp[1] * disp[1];
+    if (D >= 3) d2 = d2 + disp[2] * disp[2];
+    bool open = t < total && j != i && d2 < fp.rc2;
+    if (!__any_sync(0xffffffffu, open)) continue;
+    if (FINDER == 3) {
+      const float m[3] = {h.x - disp[0] * 0.5f, h.y - disp[1] * 0.5f, D >= 3 ? h.z - disp[2] * 0.5f : 0.f};
+      const float rsq = d2 * fp.gab_factor;
+      const BallBins<D> range(g, m, sqrtf(rsq));
+      for (int k = 0; k < kRows && __any_sync(0xffffffffu, open); ++k) {
+        const unsigned b = __shfl_sync(0xffffffffu, base, k), e1 = __shfl_sync(0xffffffffu, end, k) + b;
+        for (unsigned w0 = (k ? __shfl_sync(0xffffffffu, end, k - 1) : 0u) + b; w0 < e1; w0 += 8u) {
+          if (!__any_sync(0xffffffffu, open)) break;
+          unsigned in = 0u;  // (a row's last witness is tested again in place of those past its end)
+#pragma unroll
+          for (unsigned u = 0u; u < 8u; ++u) {
+            const unsigned w = min(w0 + u, e1 - 1u);
+            const float4 vk = sm.x[w];
+            const float e0 = vk.x - m[0], f0 = vk.y - m[1];
+            float q = e0 * e0 + f0 * f0;
+            if (D >= 3) { const float e2 = vk.z - m[2]; q = q + e2 * e2; }
+            if (q < rsq && w != i && w != j) in |= 1u << u;
+          }
+          for (; in && open; in &= in - 1u)
+            open = !range.holds(g, sm.key[min(w0 + (unsigned)__ffs(in) - 1u, e1 - 1u)]);
+        }
+      }
+    }
+    const float dist = sqrtf(d2);
+    float s[3] = {0.f, 0.f, 0.f}, bv[3] = {0.f, 0.f, 0.f}, bp[2] = {0.f, 0.f}, al[2] = {0.f, 0.f};
+    if (open) {
+      if (FORCE != 0) spring_term<D>(fp, disp, dist, s);
+      if (FORCE == 2) {
+        const float2 pj = sm.p[j];
+        polarity_terms(fp, disp, dist, pi, ti, pj, pol_trig(pj), bv, bp, al);
+      }
+    }
+    if (FORCE == 1) {
+      // (lane d adds component d; the other lanes' +0 leave a sum unchanged)
+      near[lane] = make_float4(s[0], s[1], s[2], 0.f);
+      __syncwarp();
+      const float* term = reinterpret_cast<const float*>(near) + (lane < 3u ? lane : 0u);
+#pragma unroll 8
+      for (int k = 0; k < 32; ++k) sum = sum + term[4 * k];
+      __syncwarp();
+    }
+    for (unsigned m = FORCE == 2 ? __ballot_sync(0xffffffffu, open) : 0u; m; m &= m - 1u) {
+      const int k = __ffs(m) - 1;
+#pragma unroll
+      for (int d = 0; d < D; ++d) acc.x[d] = acc.x[d] + __shfl_sync(0xffffffffu, s[d], k);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) acc.x[d] = acc.x[d] + __shfl_sync(0xffffffffu, bv[d], k);
+#pragma unroll
+      for (int d = 0; d < 2; ++d) acc.p[d] = acc.p[d] + __shfl_sync(0xffffffffu, bp[d], k);
+#pragma unroll
+      for (int d = 0; d < 2; ++d) acc.p[d] = acc.p[d] + __shfl_sync(0xffffffffu, al[d], k);
+    }
+  }
+  if (FORCE == 1)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) acc.x[d] = __shfl_sync(0xffffffffu, sum, d);
+}
+
+// One cell's sums by one warp: its candidates 32 at a time, a lane each; the
+// in-cutoff ones listed in candidate order; a lane a pair for the witness test
+// and the terms, which every lane then adds in that order.  False: more
+// neighbours than the list holds.
+template <int D, int FINDER, int FORCE>
+__device__ __forceinline__ bool small_cell(const GridP& g, const ForceP& fp, const SmallScratch& sm, unsigned i,
+                                           const uint2* rows, float4* near, Acc& acc) {
+  constexpr int kRows = D >= 3 ? 9 : 3;
+  const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  acc = Acc{{0.f, 0.f, 0.f}, {0.f, 0.f}};
+  const float4 h = sm.x[i];
+  unsigned end, base;
+  small_rows(rows, kRows, end, base);
+  const unsigned total = __shfl_sync(0xffffffffu, end, kRows - 1);
   unsigned cnt = 0u;
   for (unsigned t0 = 0u; t0 < total; t0 += 32u) {
     const unsigned t = t0 + lane;
@@ -1929,7 +2031,7 @@ static __global__ void __launch_bounds__(kSmallThreads)
     // 5. the slots of the rows of bins around the share's cells
     constexpr int kRows = D >= 3 ? 9 : 3;
     const unsigned cells = i1 - i0;
-    if (tid == 0) sm.general = 0u;
+    if (tid == 0) sm.crowded = 0u;
     for (unsigned q = tid; q < cells * kRows; q += kSmallThreads) {
       const unsigned r = q % kRows;
       const float4 v4 = sm.x[i0 + q / kRows];
@@ -1950,39 +2052,31 @@ static __global__ void __launch_bounds__(kSmallThreads)
     // 6. the cells' forces, one warp a cell
     for (unsigned c = tid >> 5; c < cells; c += kSmallThreads / 32) {
       Acc acc;
-      const bool ok = small_cell<D, FINDER, FORCE>(g, fp, sm, n, i0 + c, sm.rows + c * kRows, sm.near[tid >> 5], PA != nullptr, acc);
+      const bool ok = small_cell<D, FINDER, FORCE>(g, fp, sm, i0 + c, sm.rows + c * kRows, sm.near[tid >> 5], acc);
       if ((tid & 31u) == 0u) {
-        if (!ok) sm.list[atomicAdd(&sm.general, 1u)] = c;
+        if (!ok) sm.list[atomicAdd(&sm.crowded, 1u)] = c;
         sm.acc[c] = acc;
       }
     }
     __syncthreads();
+    if (sm.crowded) {
+      for (unsigned q = tid >> 5; q < sm.crowded; q += kSmallThreads / 32) {
+        const unsigned c = sm.list[q];
+        Acc acc;
+        small_cell_crowded<D, FINDER, FORCE>(g, fp, sm, i0 + c, sm.rows + c * kRows, sm.near[tid >> 5], acc);
+        if ((tid & 31u) == 0u) sm.acc[c] = acc;
+      }
+      __syncthreads();
+    }
+    // the bin offsets, for later steps that keep this sort
+    if (off_out && blockIdx.x == 0)
+      for (unsigned b = tid; b <= g.nbins; b += kSmallThreads) off_out[b] = first_key(sm, shift, b);
     PassArgs a = p1;
     a.X = sm.x;
     a.Bx = sm.x;
     a.P = PA ? sm.p : nullptr;
     a.Bp = a.P;
     a.Bid = sm.id;
-    // the bin offsets, for cells that take the general path or for later steps
-    // that keep this sort
-    if (sm.general || off_out) {
-      for (unsigned b = tid; b <= g.nbins; b += kSmallThreads) {
-        const unsigned e = first_key(sm, shift, b);
-        sm.off[b] = e;
-        if (off_out && blockIdx.x == 0) off_out[b] = e;
-      }
-      __syncthreads();
-      a.off = sm.off;
-      if (tid < sm.general) {
-        const unsigned c = sm.list[tid], i = i0 + c;
-        const float4 v4 = sm.x[i];
-        const float xi[3] = {v4.x, v4.y, v4.z};
-        Acc acc = {{0.f, 0.f, 0.f}, {0.f, 0.f}};
-        cell_general<D, FINDER, FORCE>(g, fp, a, n, i, xi, PA ? sm.p[i] : make_float2(0.f, 0.f), 0u, acc);
-        sm.acc[c] = acc;
-      }
-      __syncthreads();
-    }
     cluster_wait();  // every block has read the state
     if (tid < cells) {
       const unsigned i = i0 + tid;
