@@ -1226,35 +1226,56 @@ __device__ __forceinline__ void cell_general(const GridP& g, const ForceP& fp, c
 }
 
 // The naive finders' pass (FINDER 0, 2, 4: every j is a candidate), one warp
-// per CELLS cells: the lanes test 32 candidates at a time, the in-cutoff
-// lanes form their pairs' terms side by side, and the terms are added in j
-// order -- the reference's order, so the sums are those of cell_general bit
-// for bit.  A Gabriel pair's witnesses are tested by all lanes.
+// per CELLS cells: the lanes test 32 candidates at a time and the in-cutoff
+// lanes form their pairs' terms side by side and hand them over in shared
+// memory.  Lane 8 c + d adds component d of cell c, in j order -- the
+// reference's order, so the sums are those of cell_general bit for bit.  A
+// Gabriel pair's witnesses are tested by all lanes.
 // What bounds it: instruction issue and L1/L2 reads of the positions.  One
-// thread per cell (the form before) walks the n candidates in one dependent
-// chain and fills 21 of 152 SMs at 2,003 cells: 280 us a pass there.
+// thread per cell walks the n candidates in one dependent chain and fills 21 of
+// 152 SMs at 2,003 cells: 280 us a pass there.  Terms passed on by shuffles,
+// every lane adding every term, cost as many instructions a pair as forming it
+// takes a warp: with all of 60,013 cells in cutoff 74.8 ms a pass, where one
+// thread per cell takes 18.1 and this 12.2.
 constexpr int kNaiveThreads = 256;
 
 template <int D, int FINDER, int FORCE, int CELLS>
-static __global__ void __launch_bounds__(kNaiveThreads) k_pass_naive(GridP g, ForceP fp, PassArgs a) {
+static __global__ void __launch_bounds__(kNaiveThreads, FINDER == 0 && CELLS == 1 ? 5 : 4) k_pass_naive(GridP g, ForceP fp, PassArgs a) {
   static_assert(FINDER == 0 || FINDER == 2 || FINDER == 4, "the naive finders");
+  static_assert(CELLS == 1 || (FINDER == 0 && FORCE != 2), "several cells a warp: all pairs, spring laws");
   const unsigned n = a.ctr->n;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned i0 = (blockIdx.x * (kNaiveThreads / 32) + (threadIdx.x >> 5)) * CELLS;
   float xs[CELLS][3];
   float2 ps[CELLS];
   unsigned ids[CELLS];
-  Acc acc[CELLS];
 #pragma unroll
   for (int c = 0; c < CELLS; ++c) {
     const unsigned i = i0 + c;
-    const float4 v = i < n ? __ldg(&a.X[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    // (a place past the last cell is infinitely far from every cell)
+    const float4 v = i < n ? __ldg(&a.X[i]) : make_float4(INFINITY, INFINITY, INFINITY, 0.f);
     xs[c][0] = v.x; xs[c][1] = v.y; xs[c][2] = v.z;
     ids[c] = id_of(v);
     ps[c] = (FORCE == 2 && a.P && i < n) ? a.P[i] : make_float2(0.f, 0.f);
-    acc[c] = Acc{{0.f, 0.f, 0.f}, {0.f, 0.f}};
   }
-  constexpr int U = 4;  // rounds of 32 candidates in flight
+  PolTrig ti[FORCE == 2 ? CELLS : 1];
+  if (FORCE == 2)
+#pragma unroll
+    for (int c = 0; c < CELLS; ++c) ti[c] = pol_trig(ps[c]);
+  // A round's terms: for each cell its kTerms components of 32 pairs (the
+  // spring's three, with the polarity law also the bending vector and two pairs
+  // of angles).  kLine: a component's 32 places, padded so that the lanes that
+  // add different components read different banks.
+  constexpr int kTerms = FORCE == 2 ? 10 : D, kLine = 36;
+  __shared__ __align__(16) float terms_s[FORCE == 0 ? 1 : kNaiveThreads / 32 * CELLS * kTerms * kLine];
+  float* const terms = terms_s + (FORCE == 0 ? 0 : (threadIdx.x >> 5) * CELLS * kTerms * kLine);
+  const unsigned comp = lane & 7u, of = lane >> 3 < (unsigned)CELLS ? lane >> 3 : 0u;
+  // (the components in order: s, bv; bp, al: a polar lane adds two of each pair)
+  const float* const first =
+      terms + (of * kTerms + (comp < (unsigned)D ? comp : comp < 5u && FORCE == 2 ? comp + 3u : 0u)) * kLine;
+  const float* const second = first + (comp < 3u ? 3 : 2) * kLine;  // FORCE 2: added right after
+  float own = 0.f;
+  constexpr int U = CELLS == 1 && FORCE != 2 ? 4 : 2;  // rounds of 32 candidates in flight
   for (unsigned j0 = 0; j0 < (i0 < n ? n : 0u); j0 += 32u * U) {
     float4 v[U];
 #pragma unroll
@@ -1265,13 +1286,19 @@ static __global__ void __launch_bounds__(kNaiveThreads) k_pass_naive(GridP g, Fo
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const unsigned j = j0 + 32u * u + lane;
+      unsigned any = 0u, reps = 1u;  // any: lanes with a pair of one of the cells
+      unsigned accepted[CELLS];
+      float2 pj = make_float2(0.f, 0.f);
+      PolTrig tj{0.f, 0.f, 0.f, 0.f};
+      bool have = false;
 #pragma unroll
       for (int c = 0; c < CELLS; ++c) {
         const unsigned i = i0 + c;
+        accepted[c] = 0u;
         float disp[3] = {xs[c][0] - v[u].x, xs[c][1] - v[u].y, 0.f};
         float d2 = disp[0] * disp[0] + disp[1] * disp[1];
         if (D >= 3) { disp[2] = xs[c][2] - v[u].z; d2 = d2 + disp[2] * disp[2]; }
-        bool in = j < n && j != i && i < n && !(d2 >= fp.rc2);
+        bool in = j < n && j != i && !(d2 >= fp.rc2);
         unsigned bits = __ballot_sync(0xffffffffu, in);
         if (!bits) continue;
         if (FINDER == 2) {
@@ -1305,16 +1332,17 @@ static __global__ void __launch_bounds__(kNaiveThreads) k_pass_naive(GridP g, Fo
           bits = keep;
           in = (keep >> lane) & 1u;
         }
-        unsigned reps = 1u;
         if (FINDER == 4) {
           reps = in ? a.dmult[(size_t)i * a.capacity + j] : 0u;
           in = reps != 0u;
           bits = __ballot_sync(0xffffffffu, in);
         }
         if (!bits) continue;
-        float s[3] = {0.f, 0.f, 0.f}, bv[3], bp[2], al[2];
+        accepted[c] = bits;
+        any |= bits;
+        float s[3] = {0.f, 0.f, 0.f}, bv[3] = {0.f, 0.f, 0.f}, bp[2] = {0.f, 0.f}, al[2] = {0.f, 0.f};
         if (in) {
-          if (a.pairs) {
+          if (a.pairs && (CELLS == 1 || i < n)) {
             const unsigned long long at = atomicAdd(&a.ctr->pair_count, (unsigned long long)reps);
             for (unsigned r = 0; r < reps; ++r)
               if (at + r < a.pair_cap) a.pairs[at + r] = make_uint2(ids[c], id_of(v[u]));
@@ -1322,51 +1350,86 @@ static __global__ void __launch_bounds__(kNaiveThreads) k_pass_naive(GridP g, Fo
           const float dist = sqrtf(d2);
           if (FORCE != 0) spring_term<D>(fp, disp, dist, s);
           if (FORCE == 2) {
-            const float2 pj = a.P ? a.P[j] : make_float2(0.f, 0.f);
-            polarity_terms(fp, disp, dist, ps[c], pol_trig(ps[c]), pj, pol_trig(pj), bv, bp, al);
+            if (!have) {
+              if (a.P) pj = a.P[j];
+              tj = pol_trig(pj);
+              have = true;
+            }
+            polarity_terms(fp, disp, dist, ps[c], ti[c], pj, tj, bv, bp, al);
           }
         }
-        // a pair at distance zero has a +0 spring term, which leaves the sum unchanged
-        for (; bits && FORCE != 0; bits &= bits - 1u) {
-          const int src = __ffs(bits) - 1;
-          const unsigned rr = FINDER == 4 ? __shfl_sync(0xffffffffu, reps, src) : 1u;
-          float t[10];
+        // (the +0 of a lane without a pair, or of a pair at distance zero,
+        // leaves a sum unchanged that is never -0)
+        float* const t = terms + c * kTerms * kLine + lane;
+        if (FORCE != 0)
 #pragma unroll
-          for (int d = 0; d < D; ++d) t[d] = __shfl_sync(0xffffffffu, s[d], src);
-          if (FORCE == 2) {
+          for (int d = 0; d < D; ++d) t[d * kLine] = s[d];
+        if (FORCE == 2) {
 #pragma unroll
-            for (int d = 0; d < 3; ++d) t[3 + d] = __shfl_sync(0xffffffffu, bv[d], src);
+          for (int d = 0; d < 3; ++d) t[(3 + d) * kLine] = bv[d];
 #pragma unroll
-            for (int d = 0; d < 2; ++d) {
-              t[6 + d] = __shfl_sync(0xffffffffu, bp[d], src);
-              t[8 + d] = __shfl_sync(0xffffffffu, al[d], src);
-            }
+          for (int d = 0; d < 2; ++d) {
+            t[(6 + d) * kLine] = bp[d];
+            t[(8 + d) * kLine] = al[d];
           }
-          for (unsigned r = 0; r < rr; ++r) {
+        }
+      }
+      if constexpr (FORCE != 0) {
+        if (!any) continue;
+        if (FINDER != 4 && __popc(any) > 8) {
 #pragma unroll
-            for (int d = 0; d < D; ++d) acc[c].x[d] = acc[c].x[d] + t[d];
-            if (FORCE == 2) {
+          for (int c = 0; c < CELLS; ++c)
+            if (CELLS > 1 && !accepted[c])
 #pragma unroll
-              for (int d = 0; d < 3; ++d) acc[c].x[d] = acc[c].x[d] + t[3 + d];
-              acc[c].p[0] = acc[c].p[0] + t[6];
-              acc[c].p[1] = acc[c].p[1] + t[7];
-              acc[c].p[0] = acc[c].p[0] + t[8];
-              acc[c].p[1] = acc[c].p[1] + t[9];
+              for (int k = 0; k < kTerms; ++k) terms[(c * kTerms + k) * kLine + lane] = 0.f;
+          __syncwarp();
+#pragma unroll 2
+          for (int src = 0; src < 32; src += 4) {
+            const float4 t0 = *reinterpret_cast<const float4*>(first + src);
+            const float4 t1 = FORCE == 2 ? *reinterpret_cast<const float4*>(second + src) : t0;
+            own = own + t0.x;
+            if (FORCE == 2) own = own + t1.x;
+            own = own + t0.y;
+            if (FORCE == 2) own = own + t1.y;
+            own = own + t0.z;
+            if (FORCE == 2) own = own + t1.z;
+            own = own + t0.w;
+            if (FORCE == 2) own = own + t1.w;
+          }
+        } else {
+          // few pairs: the places that one of the cells has, each lane those of its own
+          __syncwarp();
+          unsigned here = accepted[0];
+#pragma unroll
+          for (int c = 1; c < CELLS; ++c)
+            if (of == (unsigned)c) here = accepted[c];
+          for (; any; any &= any - 1u) {
+            const int src = __ffs(any) - 1;
+            const float t0 = first[src], t1 = FORCE == 2 ? second[src] : 0.f;
+            const unsigned rr = FINDER == 4 ? __shfl_sync(0xffffffffu, reps, src) : here >> src & 1u;
+            for (unsigned r = 0; r < rr; ++r) {
+              own = own + t0;
+              if (FORCE == 2) own = own + t1;
             }
           }
         }
+        __syncwarp();
       }
     }
   }
   // lane c commits cell c
-  Acc mine = acc[0];
+  Acc mine = {{0.f, 0.f, 0.f}, {0.f, 0.f}};
+  if (FORCE != 0) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) mine.x[d] = __shfl_sync(0xffffffffu, own, (int)(lane & 3u) * 8 + d);
+    if (FORCE == 2)
+#pragma unroll
+      for (int d = 0; d < 2; ++d) mine.p[d] = __shfl_sync(0xffffffffu, own, (int)(lane & 3u) * 8 + 3 + d);
+  }
   float2 pi = ps[0];
 #pragma unroll
   for (int c = 1; c < CELLS; ++c)
-    if (lane == (unsigned)c) {
-      mine = acc[c];
-      pi = ps[c];
-    }
+    if (lane == (unsigned)c) pi = ps[c];
   const unsigned i = i0 + lane;
   const bool active = lane < (unsigned)CELLS && i < n;
   const float4 vi = active ? a.X[i] : make_float4(0.f, 0.f, 0.f, 0.f);

@@ -287,12 +287,17 @@ bool coop_pass(const tecs_sim* s) {
          grid_resolved(s->g, s->d.cutoff);
 }
 
-// The naive finders' pass: cells per warp.  One cell a warp fills the GPU up
-// to kNaiveOneCell cells; above, a warp takes four, which share each read of
-// the candidates' positions.
-constexpr unsigned kNaiveOneCell = 16384;
+// The naive finders' pass: cells per warp.  One cell a warp fills the GPU; many
+// cells of an all-pairs pass go four to a warp, which share each read of the
+// candidates' positions and their additions.  One and four cells a warp, cutoff
+// 1 / 4 / past all cells: 20,011 cells 0.33 / 0.67 / 1.88 and 0.40 / 0.89 / 1.82 ms;
+// 100,003 cells 7.1 / 8.9 / 43.7 and 6.2 / 8.4 / 32.1.  The polarity law (60,013
+// cells, 3.2 / 72 against 6.9 / 128 with four) and the Gabriel finder (20,011,
+// 2.4 / 57 against 3.6 / 77), whose work is in their pairs, take one.
+constexpr unsigned kNaiveOneCell = 32768;
 unsigned naive_cells(const tecs_sim* s) {
-  return s->d.finder == TECS_FINDER_NAIVE_DELAUNAY || launch_count(s) <= kNaiveOneCell ? 1u : 4u;
+  return s->d.finder == TECS_FINDER_NAIVE_ALL_PAIRS && s->d.force != TECS_FORCE_POLARITY &&
+                 launch_count(s) > kNaiveOneCell ? 4u : 1u;
 }
 
 PassFn pass_fn(const tecs_sim* s, bool sym) {
@@ -326,18 +331,18 @@ PassFn pass_fn(const tecs_sim* s, bool sym) {
   }
   PICK_SYM(3, 0) PICK_SYM(3, 2) PICK_SYM(2, 0) PICK_SYM(2, 2)
 #undef PICK_SYM
-#define PICK_NAIVE(DD, FF, CC)                                                  \
+#define PICK_NAIVE(DD, FF)                                                      \
   if (D == DD && F == FF && !sym) {                                             \
-    if (FO == 0) return k_pass_naive<DD, FF, 0, CC>;                            \
-    if (FO == 1) return k_pass_naive<DD, FF, 1, CC>;                            \
-    if (DD == 3) return k_pass_naive<3, FF, 2, CC>;                             \
+    if (FO == 0) return k_pass_naive<DD, FF, 0, 1>;                             \
+    if (FO == 1) return k_pass_naive<DD, FF, 1, 1>;                             \
+    if (DD == 3) return k_pass_naive<3, FF, 2, 1>;                              \
   }
-  if (naive_cells(s) == 1) {
-    PICK_NAIVE(3, 0, 1) PICK_NAIVE(3, 2, 1) PICK_NAIVE(3, 4, 1)
-    PICK_NAIVE(2, 0, 1) PICK_NAIVE(2, 2, 1) PICK_NAIVE(2, 4, 1)
-  } else {
-    PICK_NAIVE(3, 0, 4) PICK_NAIVE(3, 2, 4) PICK_NAIVE(2, 0, 4) PICK_NAIVE(2, 2, 4)
+  if (!sym && naive_cells(s) == 4) {
+    if (D == 3) return FO == 0 ? k_pass_naive<3, 0, 0, 4> : k_pass_naive<3, 0, 1, 4>;
+    return FO == 0 ? k_pass_naive<2, 0, 0, 4> : k_pass_naive<2, 0, 1, 4>;
   }
+  PICK_NAIVE(3, 0) PICK_NAIVE(3, 2) PICK_NAIVE(3, 4)
+  PICK_NAIVE(2, 0) PICK_NAIVE(2, 2) PICK_NAIVE(2, 4)
 #undef PICK_NAIVE
   if (F == TECS_FINDER_DELAUNAY && !sym) {
     if (D == 3 && FO == 0) return k_pass<3, 5, 0>;
