@@ -82,7 +82,7 @@ struct PassArgs {
   unsigned* cnt;
   unsigned* part;       // scan chunk totals formed while counting (count_bin), or null
   // naive Delaunay: how many times each directed pair is applied, row i at i * capacity
-  const unsigned* dmult;
+  const unsigned short* dmult;
   // Delaunay (any capacity): cell i's partners and their applications,
   // dl_row[i * kDlRow + t] = (j, reps) for t < dl_len[i], ascending j
   const uint2* dl_row;
@@ -603,7 +603,7 @@ __device__ __forceinline__ bool delaunay_inside(const float4& pm, const float* c
 }
 
 constexpr int kDelaunayThreads = 256;
-constexpr unsigned kDelaunayMaxCells = 4096;  // the pair-count table is capacity^2 x 4 bytes
+constexpr unsigned kDelaunayMaxCells = 4096;  // the pair-count table is capacity^2 x 2 bytes
 // Blocks per cell: the third points are dealt to their warps in turn, so that
 // a cell with many pairs takes no longer than its share of the GPU (with the
 // pairs dealt to four blocks the SMs waited 36 % of 2.0 ms for the last ones,
@@ -624,7 +624,7 @@ constexpr unsigned kDelaunayNear = 64;  // points near i that each simplex is te
 template <int D>
 static __global__ void __launch_bounds__(kDelaunayThreads)
 k_delaunay_mult(const float4* __restrict__ X, const Counters* __restrict__ ctr, float rc2, unsigned stride,
-                unsigned* __restrict__ mult) {  // (cleared before)
+                unsigned short* __restrict__ mult) {  // (cleared before)
   __shared__ float4 near[kDelaunayNear];  // w: the point's index
   __shared__ unsigned nnear;
   const unsigned n = ctr->n;
@@ -727,7 +727,11 @@ k_delaunay_mult(const float4* __restrict__ X, const Counters* __restrict__ ctr, 
           if (D == 3 && accepted) break;
         }
       }
-      if (lane == 0u && local) atomicAdd(&mult[(size_t)i * stride + j], local);
+      if (lane == 0u && local) {
+        // a count is below 2^16, so adding it to its half of a word carries nothing over
+        const size_t at = (size_t)i * stride + j;
+        atomicAdd(reinterpret_cast<unsigned*>(mult) + at / 2, local << (at & 1 ? 16 : 0));
+      }
     }
   }
 }

@@ -187,7 +187,7 @@ struct tecs_sim {
   unsigned *key = nullptr, *rank = nullptr, *src = nullptr, *cnt = nullptr, *off = nullptr, *part = nullptr;
   unsigned *div_parent = nullptr, *div_slot = nullptr;
   unsigned* Bid = nullptr;  // cell ids of B's slots (B.w holds the bin key)
-  unsigned* dmult = nullptr;  // naive Delaunay: applications per directed pair, capacity x capacity
+  unsigned short* dmult = nullptr;  // naive Delaunay: applications per directed pair, capacity x capacity, to whole words
   // Delaunay of any capacity: the pass's bin grid (state, counts, offsets,
   // sorted slots and positions) and each cell's partner row
   DlState* dl_st = nullptr;
@@ -509,7 +509,7 @@ int enqueue_delaunay_mult(tecs_sim* s, const PassArgs& a, int& K) {
   // applications per pair on this pass's positions, before the pass
   PROF_BEGIN(s);
   const dim3 mb(L ? L : 1, kDelaunaySplit);
-  CK(cudaMemsetAsync(s->dmult, 0, (size_t)L * s->d.capacity * 4, s->stream));
+  CK(cudaMemsetAsync(s->dmult, 0, (size_t)L * s->d.capacity * 2, s->stream));
   if (s->d.dims == 3) k_delaunay_mult<3><<<mb, kDelaunayThreads, 0, s->stream>>>(a.X, s->ctr, s->fp.rc2, s->d.capacity,
                                                                                  s->dmult);
   else k_delaunay_mult<2><<<mb, kDelaunayThreads, 0, s->stream>>>(a.X, s->ctr, s->fp.rc2, s->d.capacity, s->dmult);
@@ -930,7 +930,7 @@ int tecs_sim_create(const tecs_sim_desc* desc, tecs_sim** out) {
   ok = ok && alloc((void**)&s->key, cap * 4) && alloc((void**)&s->rank, cap * 4) && alloc((void**)&s->src, cap * 4);
   ok = ok && alloc((void**)&s->div_parent, cap * 4) && alloc((void**)&s->div_slot, cap * 4);
   if (s->binned) ok = ok && alloc((void**)&s->Bid, cap * 4);
-  if (desc->finder == TECS_FINDER_NAIVE_DELAUNAY) ok = ok && alloc((void**)&s->dmult, cap * cap * 4);
+  if (desc->finder == TECS_FINDER_NAIVE_DELAUNAY) ok = ok && alloc((void**)&s->dmult, (cap * cap + 1) / 2 * 4);
   if (desc->finder == TECS_FINDER_DELAUNAY) {
     // about two cells per bin: capacity / 2 bins suffice (dl::plan_grid)
     s->dl_maxbins = (unsigned)(cap / 2 + 64);

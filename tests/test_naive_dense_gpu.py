@@ -80,6 +80,37 @@ def test_delaunay_counts_with_every_cell_in_cutoff(dims):
     same(cells(40, dims), "naive_delaunay", 1e6)
 
 
+@pytest.mark.parametrize("n,capacity", [(41, 41), (40, 43), (64, 64)])
+@pytest.mark.parametrize("dims", [2, 3])
+def test_delaunay_table_of_half_words(dims, n, capacity):
+    # rows that start at either half of a word, and a second evaluation that
+    # finds the first one's counts
+    x = cells(n, dims)
+    s = tg.Simulation(tg.Settings(agent_count=n, capacity=capacity, cutoff_distance=1.5,
+                                  pair_finder_settings=tg.PairFinderSettings(**BOX)),
+                      dims=dims, pair_finder="naive_delaunay", integrator="euler")
+    o = oracle.Oracle(dims=dims, finder=oracle.NAIVE_DELAUNAY, cutoff=1.5, integrator=oracle.EULER, capacity=capacity, **BOX)
+    s.set_state(x)
+    o.set_state(x)
+    for _ in range(2):
+        d, _, p = s.evaluate()
+        od, _, op = o.evaluate()
+        np.testing.assert_array_equal(tg.canonical_pairs(p), tg.canonical_pairs(op))
+        np.testing.assert_array_equal(d, od)
+
+
+def test_delaunay_table_takes_two_bytes_a_pair():
+    import torch
+
+    sim(cells(64, 3), "naive_delaunay", 1.0).close()
+    before = torch.cuda.mem_get_info()[0]
+    s = sim(np.zeros((4096, 3), np.float32), "naive_delaunay", 1.0)
+    used = before - torch.cuda.mem_get_info()[0]
+    s.close()
+    # 33.6 MB, the cells' arrays (about 200 bytes each) and 2 MB pages; at four bytes 67 MB
+    assert used < 4096 * 4096 * 2 + (16 << 20)
+
+
 @pytest.mark.parametrize("cutoff", [1.5, 50.0])
 @pytest.mark.parametrize("n", [40, 321])
 def test_polarity_sums_do_not_depend_on_the_place_in_a_round(n, cutoff):
