@@ -292,7 +292,24 @@ def pass_profile(workload: str, key: str):
 
 
 def traffic_per_pass(workload: str):
-    return pass_profile(workload, "pass_dram_bytes_per_cell")
+    return pass_profile(workload, "dram_bytes_per_cell")
+
+
+# steps of a small simulation in one launch of k_step_small (kSmallSteps, csrc/tecs_gpu.cu)
+SMALL_STEPS = 32
+
+
+def launches_per_call(kernels, per_step: int, steps: int) -> int:
+    """Kernel launches of one call of `steps` steps."""
+    return -(-steps // SMALL_STEPS) if set(kernels) == {"k_step_small"} else per_step * steps
+
+
+def roofline_kernel(kernels) -> str:
+    if "k_step_small" in kernels:
+        # profiled one step a launch: the launch figures are those of a step
+        return (f"one Euler step of k_step_small (bin sort + pair finding + force + integrator; a launch holds up to "
+                f"{SMALL_STEPS} steps, the launch figures are per step)")
+    return "force pass (k_pass_*: pair finding + force + fused integrator epilogue)"
 
 
 def cpu_steps(w, n, mn, mx, x, p, steps, threads, budget_s):
@@ -418,8 +435,7 @@ def run_gb300(args):
     torch.cuda.synchronize()
     value = cell_steps_all / total_s
     kpl = sim.kernels_per_step()
-    # small Euler steps (k_step_small): one launch takes up to 256 of a call's steps
-    launches = -(-chunk // 256) if set(kern) == {"k_step_small"} else kpl * chunk
+    launches = launches_per_call(kern, kpl, chunk)
 
     # End to end through the C ABI with host buffers: every step uploads the
     # state from pinned host memory, steps, and downloads the new state.
@@ -498,13 +514,10 @@ def run_gb300(args):
     pass_launch_s = share * timed_step_s / max(launches_per_step, 1e-9)
     bytes_per_launch = pass_bytes / max(pass_launches, 1)
     achieved = bytes_per_launch * (n_avg / n_prof) / pass_launch_s / 1e9 if pass_launch_s else float("nan")
-    # (the "pass_" figures are those of the pass before its warps shared the cells' work)
-    tpc = pass_profile(args.workload, "dram_bytes_per_cell") or traffic_per_pass(args.workload)
+    tpc = traffic_per_pass(args.workload)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                 "traffic": (tpc * n_avg if tpc else None),
-                "kernel": ("Euler steps in one launch (k_step_small: bin sort + pair finding + force + integrator)"
-                           if "k_step_small" in kern else
-                           "force pass (k_pass_*: pair finding + force + fused integrator epilogue)"),
+                "kernel": roofline_kernel(kern),
                 "bytes_per_launch": bytes_per_launch * n_avg / n_prof,
                 "peak_kind": f"{peak_kind} hbm_gbs", "avg_launch_ms": 1e3 * pass_launch_s,
                 "avg_launch_ms_basis": "the pass's share of the profiled step (per-kernel CUDA events) times "
