@@ -170,32 +170,6 @@ __device__ __forceinline__ void order_points(const Warp& w, LocalScratch<LOC>& s
   __syncwarp();
 }
 
-// The circumcentre of the cell at pi and three others, relative to the cell.
-__device__ __forceinline__ void tet_centre(const Grid& g, const double* pi, unsigned ia, unsigned ib, unsigned ic,
-                                           double* x) {
-  double a[3], b[3], c[3];
-  load(g.P[ia], a);
-  load(g.P[ib], b);
-  load(g.P[ic], c);
-  double ha = 0.0, hb = 0.0, hc = 0.0;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    a[d] -= pi[d];
-    b[d] -= pi[d];
-    c[d] -= pi[d];
-    ha += a[d] * a[d];
-    hb += b[d] * b[d];
-    hc += c[d] * c[d];
-  }
-  double bc[3], ca[3], ab[3];
-  cross3(b, c, bc);
-  cross3(c, a, ca);
-  cross3(a, b, ab);
-  const double inv = 0.5 / (a[0] * bc[0] + a[1] * bc[1] + a[2] * bc[2]);
-#pragma unroll
-  for (int d = 0; d < 3; ++d) x[d] = (ha * bc[d] + hb * ca[d] + hc * ab[d]) * inv;
-}
-
 // The circumcentres of the listed tetrahedra, and whether every gathered point
 // lies outside their spheres with certainty.
 template <int LOC>
@@ -208,27 +182,19 @@ __device__ __forceinline__ bool verify_tets(const Warp& w, const Grid& g, unsign
     const unsigned t = t0 + w.lane();
     const ushort4 q = sc.tet[t < m ? t : t0];
     const bool closed = q.z != kNoEnd;
-    double xd[3];
-    tet_centre(g, pi, sc.id[q.x], sc.id[q.y], sc.id[closed ? q.z : q.x], xd);
+    double xd[3], thin2;
+    tet_centre(pi, g.P[sc.id[q.x]], g.P[sc.id[q.y]], g.P[sc.id[closed ? q.z : q.x]], xd, thin2);
     const float x = (float)xd[0], y = (float)xd[1], z = (float)xd[2];
     const float r2 = x * x + y * y + z * z;
     if (t < m) sc.cen[t] = make_float4(x, y, z, r2);
-    if (closed && !(r2 < 2.5e11f * rho * rho)) bad = true;
+    if (closed && !(r2 < 2.5e11f * rho * rho && thin2 < kThin * kThin)) bad = true;
     const float m0 = kPowerX * r2;
     for (unsigned k = 0; k < n; ++k) {
       const float4 v = sc.p[k];
       const float pw = v.w - (x * v.x + y * v.y + z * v.z);
       if (closed && !(pw > kPowerV * v.w + m0) && k != q.x && k != q.y && k != q.z) {
         // too near for float: once more in double
-        double pd[3], h = 0.0, dt = 0.0, xx = 0.0;
-        load(g.P[sc.id[k]], pd);
-        for (int d = 0; d < 3; ++d) {
-          pd[d] -= pi[d];
-          h += pd[d] * pd[d];
-          dt += pd[d] * xd[d];
-          xx += xd[d] * xd[d];
-        }
-        if (!(0.5 * h - dt > 1.0e-11 * (h + xx))) bad = true;
+        if (!sphere_leaves_out(pi, xd, thin2, g.P[sc.id[k]])) bad = true;
       }
     }
     if (__any_sync(0xffffffffu, bad)) return false;
@@ -285,10 +251,10 @@ __device__ __forceinline__ int verify_far(const Warp& w, const Grid& g, unsigned
     // in float, and where a cell is too near to tell, once more in double
     for (int dbl = 0; dbl < 2; ++dbl) {
       bool doubt = false;
-      double xd[3] = {0.0, 0.0, 0.0}, xx = 0.0;
+      double xd[3] = {0.0, 0.0, 0.0}, thin2 = 0.0, margin = 0.0;
       if (dbl && closed) {
-        tet_centre(g, pi, ia, ib, ic, xd);
-        xx = xd[0] * xd[0] + xd[1] * xd[1] + xd[2] * xd[2];
+        tet_centre(pi, g.P[ia], g.P[ib], g.P[ic], xd, thin2);
+        margin = sphere_margin(thin2);
       }
       auto test = [&](unsigned e, const Pt& p) {
         if (e == i || e == ia || e == ib || e == ic) return true;
@@ -309,7 +275,8 @@ __device__ __forceinline__ int verify_far(const Warp& w, const Grid& g, unsigned
           const double* to = closed ? xd : nn;
           const double dt = v[0] * to[0] + v[1] * to[1] + v[2] * to[2];
           const double pw = closed ? 0.5 * vv - dt : -dt;
-          const double lim = closed ? 1.0e-11 * (vv + xx) : 1.0e-13 * slack * sqrt(vv);
+          const double xx = xd[0] * xd[0] + xd[1] * xd[1] + xd[2] * xd[2];
+          const double lim = closed ? margin * (vv + xx) : 1.0e-13 * slack * sqrt(vv);
           out = pw > lim;
           in = pw < -lim;
           depth = (float)-pw;

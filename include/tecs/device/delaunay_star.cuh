@@ -554,6 +554,44 @@ TECS_DL_CALL bool cuts_cross(const P& pi, const P& pj, const P& pk, const P& ph,
   return (t[1] - t[0]) * err.len > e[0] + e[1];
 }
 
+// The circumcentre x of the cell at pi and three others, relative to the cell;
+// thin2: (|a| |b| |c| / det)^2 of the three relative positions, by which rounding
+// is enlarged: x is off by at most 2^-53 thin (15 max |a| + 8 |x|).
+template <class P>
+TECS_DL_HD void tet_centre(const double* pi, const P& pa, const P& pb, const P& pc, double* x, double& thin2) {
+  const double a[3] = {pa.x - pi[0], pa.y - pi[1], pa.z - pi[2]}, b[3] = {pb.x - pi[0], pb.y - pi[1], pb.z - pi[2]},
+               c[3] = {pc.x - pi[0], pc.y - pi[1], pc.z - pi[2]};
+  double ha = 0.0, hb = 0.0, hc = 0.0;
+  for (int d = 0; d < 3; ++d) {
+    ha += a[d] * a[d];
+    hb += b[d] * b[d];
+    hc += c[d] * c[d];
+  }
+  const double bc[3] = {b[1] * c[2] - b[2] * c[1], b[2] * c[0] - b[0] * c[2], b[0] * c[1] - b[1] * c[0]};
+  const double ca[3] = {c[1] * a[2] - c[2] * a[1], c[2] * a[0] - c[0] * a[2], c[0] * a[1] - c[1] * a[0]};
+  const double ab[3] = {a[1] * b[2] - a[2] * b[1], a[2] * b[0] - a[0] * b[2], a[0] * b[1] - a[1] * b[0]};
+  const double det = a[0] * bc[0] + a[1] * bc[1] + a[2] * bc[2];
+  const double inv = 0.5 / det;
+  for (int d = 0; d < 3; ++d) x[d] = (ha * bc[d] + hb * ca[d] + hc * ab[d]) * inv;
+  thin2 = 4.0 * ha * inv * hb * inv * hc;
+}
+
+// Tetrahedra thinner than this are not decided by their centre: at 2^-53 thin its
+// error stays far below that of a float test of a point against the sphere.
+constexpr double kThin = 1.0e6;
+
+// The share of |v|^2 + |x|^2 that a point's power |v|^2 / 2 - x.v in a sphere has
+// to exceed to be certain: the centre's error (with max |a| <= 2 |x|) moves it by
+// up to 19 2^-53 thin of that, the point's own products by less than 1e-15.
+TECS_DL_HD double sphere_margin(double thin2) { return 1.0e-11 + 4.0e-15 * sqrt(thin2); }
+
+template <class P>
+TECS_DL_HD bool sphere_leaves_out(const double* pi, const double* x, double thin2, const P& p) {
+  const double v[3] = {p.x - pi[0], p.y - pi[1], p.z - pi[2]};
+  const double vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2], xx = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+  return 0.5 * vv - (v[0] * x[0] + v[1] * x[1] + v[2] * x[2]) > sphere_margin(thin2) * (vv + xx);
+}
+
 // 2-D: every entry within distance del of the line through o with unit
 // normal nrm (and a few just outside): each row of bins cut to the band.
 template <class W, class F, class R>

@@ -10,7 +10,12 @@
 //     cut in float as the search does and in double: prints
 //     "<set> <unit of length> <lines without a rest in float> <looked at in double>
 //     <doubtful> <wrong>",
-//     wrong being those called certain of which double leaves something.
+//     wrong being those called certain of which more bits leave something.
+//   delaunay_margins_host spheres
+//     tetrahedra from thin to regular, most of them with five or more points on
+//     their sphere but for rounding: prints "<refused> <outside>" and the five
+//     positions (the cell, three others, a fifth), in which outside says that
+//     the fifth is certainly outside of the first four's sphere.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -194,8 +199,44 @@ static int lines() {
   return 0;
 }
 
+static int spheres() {
+  std::mt19937 rng(11);
+  std::normal_distribution<double> nd(0.0, 1.0);
+  std::uniform_real_distribution<double> u11(-1.0, 1.0);
+  for (int t = 0; t < 6000; ++t) {
+    // corners of a turned and shifted unit cube, off by the jitter
+    const double jitter = t % 3 == 0 ? 0.0 : t % 3 == 1 ? 1e-6 : 1e-3;
+    double q[4], len = 0.0, shift[3];
+    for (double& v : q) { v = nd(rng); len += v * v; }
+    for (double& v : q) v /= std::sqrt(len);
+    for (double& v : shift) v = 3.0 * u11(rng);
+    const double r[3][3] = {
+        {1 - 2 * (q[2] * q[2] + q[3] * q[3]), 2 * (q[1] * q[2] - q[0] * q[3]), 2 * (q[1] * q[3] + q[0] * q[2])},
+        {2 * (q[1] * q[2] + q[0] * q[3]), 1 - 2 * (q[1] * q[1] + q[3] * q[3]), 2 * (q[2] * q[3] - q[0] * q[1])},
+        {2 * (q[1] * q[3] - q[0] * q[2]), 2 * (q[2] * q[3] + q[0] * q[1]), 1 - 2 * (q[1] * q[1] + q[2] * q[2])}};
+    unsigned pick[5] = {0, 1, 2, 3, 4 + (unsigned)(rng() % 4)};  // the face z = 0, and a corner above it
+    if (t % 2) pick[3] = 4 + (unsigned)(rng() % 4), pick[4] = 3;  // or a fat one, and the face's last corner
+    Pt p[5];
+    for (int k = 0; k < 5; ++k) {
+      double c[3], w[3];
+      for (int d = 0; d < 3; ++d) c[d] = ((pick[k] >> d) & 1u) + jitter * nd(rng);
+      for (int d = 0; d < 3; ++d) w[d] = r[d][0] * c[0] + r[d][1] * c[1] + r[d][2] * c[2] + shift[d];
+      p[k] = Pt{(float)w[0], (float)w[1], (float)w[2], 0.f};
+    }
+    const double pi[3] = {p[0].x, p[0].y, p[0].z};
+    double x[3], thin2;
+    tet_centre(pi, p[1], p[2], p[3], x, thin2);
+    const bool refused = !(thin2 < kThin * kThin);
+    std::printf("%d %d", refused ? 1 : 0, !refused && sphere_leaves_out(pi, x, thin2, p[4]) ? 1 : 0);
+    for (const Pt& v : p) std::printf(" %.9g %.9g %.9g", v.x, v.y, v.z);
+    std::printf("\n");
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   if (argc == 2 && !std::strcmp(argv[1], "normals")) return normals();
   if (argc == 2 && !std::strcmp(argv[1], "lines")) return lines();
+  if (argc == 2 && !std::strcmp(argv[1], "spheres")) return spheres();
   return 2;
 }

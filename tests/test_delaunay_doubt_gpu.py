@@ -2,8 +2,9 @@
 
 Rows have to be the host walk's (tests/cpp/delaunay_star_host.cpp), pair by
 pair, whichever of the searches takes a cell: hull edges that carry cells
-nearly on one line (faces too thin for a float normal), and cells in other
-units of length than about one cell a unit.
+nearly on one line (faces too thin for a float normal), cells in other units
+of length than about one cell a unit, and turned lattices, whose spheres hold
+eight cells but for rounding.
 """
 import numpy as np
 import pytest
@@ -50,3 +51,12 @@ def test_units_of_length(host_search, kind, unit):  # noqa: F811
     rows = found(x, cutoff)
     assert rows == expected(host_search, x, cutoff)
     assert len(rows) > 3 * len(x)
+
+
+@pytest.mark.parametrize("jitter", [0.0, 1e-7, 1e-5])
+def test_turned_lattices(host_search, jitter):  # noqa: F811
+    rng = np.random.default_rng(3)
+    turn = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+    x = np.stack(np.meshgrid(*[np.arange(10)] * 3, indexing="ij"), -1).reshape(-1, 3) + rng.normal(0, 1.0, (1000, 3)) * jitter
+    x = (x @ turn.T).astype(np.float32)
+    assert found(x, 1.2) == expected(host_search, x, 1.2)
