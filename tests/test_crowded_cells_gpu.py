@@ -1,5 +1,6 @@
 """Cells with many neighbours and the polarity law on a GB300, one path against another.
 
+Cells among many candidates with few of them in cutoff, against the oracle.
 Densities at which a warp's pairs fill the pool several times (about 4.5
 cells a unit volume), lists overflow into the general path (9 and 30) and the
 small steps' lists do (64 neighbours).  Runs have to be bit-identical: small
@@ -15,6 +16,7 @@ import os
 import numpy as np
 import pytest
 
+import oracle
 import tecs_gb300 as tg
 from tecs_gb300 import workloads as wl
 from tecs_gb300.engine import Engine, bins_needed
@@ -130,3 +132,26 @@ def test_engine_polarity_runs_are_the_plain_ones(finder):
         np.testing.assert_array_equal(xe, xp)
         np.testing.assert_array_equal(pe, pp)
     eng.close()
+
+
+@pytest.mark.parametrize("clump", [70, 80, 170, 190, 700])
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("finder", ["binned_all_pairs", "binned_gabriel"])
+def test_lone_cells_beside_a_clump(finder, dims, clump):
+    # a clump in the corner of one bin: the cells of the bins around it have it
+    # among their candidates, out of cutoff for most
+    rng = np.random.default_rng(6)
+    x = np.concatenate([rng.random((clump, dims)) * 0.1, rng.random((60, dims)) * 4]).astype(np.float32)
+    box = dict(min_bounds=(0.0,) * 3, max_bounds=(4.0,) * 3)
+    s = tg.Simulation(tg.Settings(agent_count=len(x), capacity=len(x), pair_finder_settings=tg.PairFinderSettings(**box)),
+                      dims=dims, pair_finder=finder, integrator="heun")
+    o = oracle.Oracle(dims=dims, finder=getattr(oracle, finder.upper()), integrator=oracle.HEUN, capacity=len(x), **box)
+    s.set_state(x)
+    o.set_state(x)
+    d, _, pairs = s.evaluate()
+    od, _, opairs = o.evaluate()
+    np.testing.assert_array_equal(tg.canonical_pairs(pairs), tg.canonical_pairs(opairs))
+    np.testing.assert_array_equal(d, od)
+    s.take_step(0.001, 2)
+    o.step(0.001, 2)
+    np.testing.assert_array_equal(s.get_state()[0], o.get_state()[0])
