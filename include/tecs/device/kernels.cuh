@@ -609,6 +609,10 @@ constexpr unsigned kDelaunayMaxCells = 4096;  // the pair-count table is capacit
 // pairs dealt to four blocks the SMs waited 36 % of 2.0 ms for the last ones,
 // 400 cells in 3-D).
 constexpr unsigned kDelaunaySplit = 16;
+// Up to so many cells a block takes a cell by itself and writes its row, without
+// the clearing of the table before: launches are what such a call costs (2 cells
+// 8.9 us a step against 13.0; past 10 cells in space the one block takes longer).
+constexpr unsigned kDelaunayOne = 8;
 constexpr unsigned kDelaunayNear = 64;  // points near i that each simplex is tested against first
 
 // Every simplex is an existence test over all points: one point inside rejects
@@ -624,13 +628,14 @@ constexpr unsigned kDelaunayNear = 64;  // points near i that each simplex is te
 template <int D>
 static __global__ void __launch_bounds__(kDelaunayThreads)
 k_delaunay_mult(const float4* __restrict__ X, const Counters* __restrict__ ctr, float rc2, unsigned stride,
-                unsigned short* __restrict__ mult) {  // (cleared before)
+                unsigned short* __restrict__ mult) {  // (cleared before, unless a block takes a cell by itself)
   __shared__ float4 near[kDelaunayNear];  // w: the point's index
-  __shared__ unsigned nnear;
+  __shared__ unsigned nnear, row[kDelaunayOne];
   const unsigned n = ctr->n;
-  const unsigned i = blockIdx.x;
+  const unsigned i = blockIdx.x, split = gridDim.y;
   if (i >= n) return;
   const unsigned t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+  if (t < kDelaunayOne) row[t] = 0u;
   const float4 pi = __ldg(&X[i]);
   const float li = sq_len<D>(pi);
   const float ci[3] = {pi.x, pi.y, pi.z};
@@ -685,7 +690,7 @@ k_delaunay_mult(const float4* __restrict__ X, const Counters* __restrict__ ctr, 
       const float lj = sq_len<D>(pj);
       unsigned local = 0;
       const unsigned items = D == 3 ? n : (n + 31u) / 32u;
-      for (unsigned q = blockIdx.y + warp * kDelaunaySplit; q < items; q += kDelaunayThreads / 32 * kDelaunaySplit) {
+      for (unsigned q = blockIdx.y + warp * split; q < items; q += kDelaunayThreads / 32 * split) {
         if (D == 3 && (q == i || q == j)) continue;
         const float4 pq = D == 3 ? __ldg(&X[q]) : pj;
         const float lq = sq_len<3>(pq);
@@ -727,12 +732,18 @@ k_delaunay_mult(const float4* __restrict__ X, const Counters* __restrict__ ctr, 
           if (D == 3 && accepted) break;
         }
       }
-      if (lane == 0u && local) {
+      if (lane == 0u && local && split == 1u) {
+        atomicAdd(&row[j], local);
+      } else if (lane == 0u && local) {
         // a count is below 2^16, so adding it to its half of a word carries nothing over
         const size_t at = (size_t)i * stride + j;
         atomicAdd(reinterpret_cast<unsigned*>(mult) + at / 2, local << (at & 1 ? 16 : 0));
       }
     }
+  }
+  if (split == 1u) {
+    __syncthreads();
+    if (t < n) mult[(size_t)i * stride + t] = (unsigned short)row[t];
   }
 }
 

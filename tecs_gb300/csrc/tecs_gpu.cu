@@ -508,8 +508,8 @@ int enqueue_delaunay_mult(tecs_sim* s, const PassArgs& a, int& K) {
   const unsigned L = launch_count(s);
   // applications per pair on this pass's positions, before the pass
   PROF_BEGIN(s);
-  const dim3 mb(L ? L : 1, kDelaunaySplit);
-  CK(cudaMemsetAsync(s->dmult, 0, (size_t)L * s->d.capacity * 2, s->stream));
+  const dim3 mb(L ? L : 1, L <= kDelaunayOne ? 1 : kDelaunaySplit);
+  if (L > kDelaunayOne) CK(cudaMemsetAsync(s->dmult, 0, (size_t)L * s->d.capacity * 2, s->stream));
   if (s->d.dims == 3) k_delaunay_mult<3><<<mb, kDelaunayThreads, 0, s->stream>>>(a.X, s->ctr, s->fp.rc2, s->d.capacity,
                                                                                  s->dmult);
   else k_delaunay_mult<2><<<mb, kDelaunayThreads, 0, s->stream>>>(a.X, s->ctr, s->fp.rc2, s->d.capacity, s->dmult);

@@ -80,11 +80,11 @@ def test_delaunay_counts_with_every_cell_in_cutoff(dims):
     same(cells(40, dims), "naive_delaunay", 1e6)
 
 
-@pytest.mark.parametrize("n,capacity", [(41, 41), (40, 43), (64, 64)])
+@pytest.mark.parametrize("n,capacity", [(1, 1), (3, 3), (5, 9), (8, 8), (8, 9), (9, 9), (41, 41), (40, 43), (64, 64)])
 @pytest.mark.parametrize("dims", [2, 3])
 def test_delaunay_table_of_half_words(dims, n, capacity):
-    # rows that start at either half of a word, and a second evaluation that
-    # finds the first one's counts
+    # rows that start at either half of a word, up to 8 cells written by one
+    # block each, and a second evaluation that finds the first one's counts
     x = cells(n, dims)
     s = tg.Simulation(tg.Settings(agent_count=n, capacity=capacity, cutoff_distance=1.5,
                                   pair_finder_settings=tg.PairFinderSettings(**BOX)),
