@@ -940,8 +940,9 @@ static __global__ void __launch_bounds__(dl::kLocalThreads)
   }
 }
 
-// The cells that the local search was not certain of: the walk in double, one
-// warp per cell, the lanes sharing each search's entries (dl::Warp).
+// The cells that the local search was not certain of (all: every cell, in bin
+// order): the walk in double, one warp per cell, the lanes sharing each search's
+// entries (dl::Warp).
 template <int D>
 static __global__ void __launch_bounds__(kDlThreads) k_dl_mult(const float4* __restrict__ X, Counters* __restrict__ ctr,
                                                                DlState* __restrict__ st,
@@ -949,7 +950,7 @@ static __global__ void __launch_bounds__(kDlThreads) k_dl_mult(const float4* __r
                                                                const unsigned* __restrict__ idx,
                                                                const float4* __restrict__ sp, float rc2,
                                                                uint2* __restrict__ row, unsigned* __restrict__ len,
-                                                               const unsigned* __restrict__ in) {
+                                                               const unsigned* __restrict__ in, bool all) {
   // the warp's star and candidate lists: one copy, in shared memory
   __shared__ __align__(16) unsigned char scratch[(kDlThreads / 32) * sizeof(dl::Scratch)];
   dl::Scratch& sc = reinterpret_cast<dl::Scratch*>(scratch)[threadIdx.x >> 5];
@@ -957,7 +958,7 @@ static __global__ void __launch_bounds__(kDlThreads) k_dl_mult(const float4* __r
   unsigned *oj = out_j[threadIdx.x >> 5], *orp = out_r[threadIdx.x >> 5];
   const dl::Grid g = dl_grid(X, ctr, st, off, idx, sp, rc2);
   const dl::Warp lanes;
-  const unsigned count = st->left[1];
+  const unsigned count = all ? g.n : st->left[1];
   for (;;) {
     unsigned at = 0u;
     if (lanes.leader()) at = atomicAdd(&st->taken[2], 1u);

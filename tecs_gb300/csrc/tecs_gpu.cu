@@ -457,6 +457,11 @@ int enqueue_rebuild(tecs_sim* s, int& K, bool run_count) {
 // Blocks of the Delaunay finder's searches: 8 an SM.
 constexpr unsigned kDlBlocks = 152 * 8;
 
+// Up to so many cells every cell is walked: most lie on the hull, where the local
+// search is in doubt, and costs two launches (5 cells in space 183 us against 175,
+// one cell 38 against 30).
+constexpr unsigned kDlWalk2 = 8, kDlWalk3 = 6;
+
 // The Delaunay finder of any capacity: bin grid of the pass's positions, then
 // every cell's partner row.
 int enqueue_delaunay_star(tecs_sim* s, const PassArgs& a, int& K) {
@@ -482,6 +487,10 @@ int enqueue_delaunay_star(tecs_sim* s, const PassArgs& a, int& K) {
   const unsigned lb = std::min(ceil_div(L ? L : 1, dl::kLocalThreads / 32), kDlBlocks);
   const unsigned mb = std::min(ceil_div(L ? L : 1, kDlThreads / 32), kDlBlocks);
   unsigned *l0 = s->dl_list, *l1 = l0 + s->d.capacity;
+#define DL_MULT(DD, list, all)                                                                                       \
+  k_dl_mult<DD><<<mb, kDlThreads, 0, s->stream>>>(a.X, s->ctr, s->dl_st, s->dl_off, s->dl_idx, s->dl_sp, s->fp.rc2,  \
+                                                  s->dl_row, s->dl_len, list, all);                                  \
+  PROF_END(s, "k_dl_mult")
 #define DL_PASS(DD)                                                                                                  \
   k_dl_local<DD, 0><<<lb, dl::kLocalThreads, 0, s->stream>>>(a.X, s->ctr, s->dl_st, s->dl_off, s->dl_idx, s->dl_sp,  \
                                                              s->fp.rc2, s->dl_row, s->dl_len, s->dl_idx, l0);        \
@@ -491,14 +500,19 @@ int enqueue_delaunay_star(tecs_sim* s, const PassArgs& a, int& K) {
                                                              s->fp.rc2, s->dl_row, s->dl_len, l0, l1);               \
   PROF_END(s, "k_dl_local_far");                                                                                     \
   PROF_BEGIN(s);                                                                                                     \
-  k_dl_mult<DD><<<mb, kDlThreads, 0, s->stream>>>(a.X, s->ctr, s->dl_st, s->dl_off, s->dl_idx, s->dl_sp, s->fp.rc2,  \
-                                                  s->dl_row, s->dl_len, l1);                                         \
-  PROF_END(s, "k_dl_mult")
+  DL_MULT(DD, l1, false)
   PROF_BEGIN(s);
-  if (d3) { DL_PASS(3); }
-  else { DL_PASS(2); }
+  if (L <= (d3 ? kDlWalk3 : kDlWalk2)) {
+    if (d3) { DL_MULT(3, s->dl_idx, true); }
+    else { DL_MULT(2, s->dl_idx, true); }
+    K += 1;
+  } else {
+    if (d3) { DL_PASS(3); }
+    else { DL_PASS(2); }
+    K += 3;
+  }
+#undef DL_MULT
 #undef DL_PASS
-  K += 3;
   CK(cudaGetLastError());
   return 0;
 }

@@ -60,3 +60,12 @@ def test_turned_lattices(host_search, jitter):  # noqa: F811
     x = np.stack(np.meshgrid(*[np.arange(10)] * 3, indexing="ij"), -1).reshape(-1, 3) + rng.normal(0, 1.0, (1000, 3)) * jitter
     x = (x @ turn.T).astype(np.float32)
     assert found(x, 1.2) == expected(host_search, x, 1.2)
+
+
+@pytest.mark.parametrize("cutoff", [0.7, 1e3])
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 6, 7, 8, 9, 10])
+def test_a_few_cells(host_search, n, dims, cutoff):  # noqa: F811
+    # walked all (up to six in space, eight in the plane) or searched first
+    x = np.ascontiguousarray(wl.ball(n, 3)[:, :dims])
+    assert found(x, cutoff) == expected(host_search, x, cutoff)
