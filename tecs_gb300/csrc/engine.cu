@@ -148,6 +148,10 @@ static __global__ void k_eorder_gather(const unsigned* __restrict__ off, unsigne
 // POL: some resident simulation carries polarity; spring-only engines use the
 // instance without the polarity law's terms.
 // TB: threads per block (64, 96 or 128; the autotuner's choice).
+// Resident threads an SM: 768 for the spring laws leave 80 registers.  With 896
+// (72 registers) ordinary ensembles gain 1 % (32 x 20,000 cells 215 against 218
+// us a step), and crowded cells on the general path lose 4 to 7 % to the form
+// before (8 x 5,000 cells at nine a bin 3.03 against 2.39 ms, 2.91 before).
 #define TECS_NO_ROW kNoRow
 #define TECS_LOAD(p) __ldg(p)
 #define TECS_ROW_SLOTS(N, lo, hi) row_slots<N>(off, lo, hi)
@@ -162,7 +166,7 @@ static __global__ void k_eorder_gather(const unsigned* __restrict__ off, unsigne
 #define TECS_CAPTURE(c, jj)
 
 template <int PASS, bool POL, int TB>
-static __global__ void __launch_bounds__(TB, (POL ? 672 : 896) / TB) k_epass(EngArgs e) {
+static __global__ void __launch_bounds__(TB, (POL ? 672 : 768) / TB) k_epass(EngArgs e) {
   constexpr int D = 3;
   __shared__ unsigned hsim[TB];
   const unsigned n = e.off[e.nb_total];
