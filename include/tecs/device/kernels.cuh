@@ -751,7 +751,7 @@ k_delaunay_mult(const float4* __restrict__ X, const Counters* __restrict__ ctr, 
 // Delaunay finder for any capacity (tecs/device/delaunay_star.cuh).  Before
 // each pass: the bounding box of the pass's positions, a bin grid of about
 // two cells per bin, a counting sort into it, then each cell's partners and
-// multiplicities (k_dl_mult, one thread per cell).  The pass applies each
+// multiplicities (k_dl_local and k_dl_mult, one warp per cell).  The pass applies each
 // listed pair reps times in ascending j, as FINDER 4 does.
 constexpr unsigned kDlRow = 64;  // partners per cell
 constexpr int kDlThreads = 64;
@@ -1771,7 +1771,8 @@ static __global__ void __launch_bounds__(kCoopThreads<FORCE>, kCoopBlocks)
 // The cluster size is set at launch (16 blocks: past the portable 8, opted
 // into per kernel).
 constexpr int kSmallCtas = 16;
-constexpr unsigned kSmallCells = kSmallCtas * kPassThreads;
+constexpr int kSmallShare = 96;  // cells of a block, at most
+constexpr unsigned kSmallCells = kSmallCtas * kSmallShare;
 constexpr unsigned kSmallBins = 16384;
 constexpr int kSmallThreads = 1024;
 constexpr unsigned kSmallGroups = 2048;                         // of the coarse histogram, four a thread of the scan
@@ -1787,10 +1788,10 @@ struct SmallScratch {
   unsigned key[kSmallCells], id[kSmallCells]; // sorted
   __align__(16) unsigned coarse[kSmallGroups + 4];  // start of each group
   unsigned wsum[kSmallThreads / 32];
-  uint2 rows[kPassThreads * 9];               // the share's rows of bins: their slots
+  uint2 rows[kSmallShare * 9];                // the share's rows of bins: their slots
   float4 near[kSmallThreads / 32][kSmallNear];
-  Acc acc[kPassThreads];                      // the share's sums
-  unsigned crowded, list[kPassThreads];       // cells of more neighbours than a list holds
+  Acc acc[kSmallShare];                       // the share's sums
+  unsigned crowded, list[kSmallShare];        // cells of more neighbours than a list holds
 };
 
 // The arrive half of the cluster's barrier and the wait half.

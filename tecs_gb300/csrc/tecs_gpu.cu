@@ -1082,8 +1082,8 @@ int tecs_sim_step(tecs_sim* s, double dt, int n_steps) {
   if (small_step_ok(s) && s->d.rebuild_every_n <= 1 && !s->profiling) {
     // every step sorts the cells anew: many steps a launch (at most
     // kSmallSteps)
-    for (int done = 0; done < n_steps; done += kSmallSteps)
-      if (launch_small(s, (float)dt, dt, std::min(kSmallSteps, n_steps - done))) return -1;
+    for (int left = n_steps; left > 0; left -= kSmallSteps)
+      if (launch_small(s, (float)dt, dt, std::min(kSmallSteps, left))) return -1;
     if (n_steps > 0) {
       s->step_count = 1;
       s->last_kernels = 1;
