@@ -914,7 +914,7 @@ __device__ __forceinline__ dl::Grid dl_grid(const float4* X, const Counters* ctr
 // its bounding box), enough for 97 % of the interior cells (spheres of 1.4 cell
 // spacings); in 2-D 2.25 bins hold about 40, enough for all but the hull.
 template <int D, int LEVEL>
-static __global__ void __launch_bounds__(dl::kLocalThreads)
+static __global__ void __launch_bounds__(dl::kLocalThreads, LEVEL == 0 ? 6 : 5)
     k_dl_local(const float4* __restrict__ X, const Counters* __restrict__ ctr, DlState* __restrict__ st,
                const unsigned* __restrict__ off, const unsigned* __restrict__ idx, const float4* __restrict__ sp,
                float rc2, uint2* __restrict__ row, unsigned* __restrict__ len, const unsigned* __restrict__ in,
