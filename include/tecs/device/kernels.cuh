@@ -1164,13 +1164,12 @@ __device__ __forceinline__ void pass_epilogue(const GridP& g, const PassArgs& a,
 // restriction on k exactly (binned_gabriel.hpp:142-207).  A cell with more
 // than kMaxNb neighbours takes the general path.
 constexpr int kMaxNb = 24;     // (4 on average at one cell per bin, 12 in packed tissue; a count is a class: at most 31)
-// Candidates in the bins around a cell past which it takes the general path
-// unwalked: a cutoff of one bin holds 0.155 of them in space (0.35 in the plane),
-// and at 27 neighbours seven cells in ten have more than kMaxNb.  200,000 cells
-// at nine a bin, all-pairs, a Heun step: 766 us with every cell walked to the
-// end first, 674 with this, 718 with a thread a cell throughout.
-template <int D>
-constexpr int kCrowd = D >= 3 ? 176 : 76;
+// Candidates in a z-plane of the bins around a cell past which it takes the
+// general path unwalked: about 33 of 3 x 72 are in cutoff in space (0.155 of
+// them) and 25 of 72 in the plane (0.35).  200,000 cells at nine a bin,
+// all-pairs, a Heun step: 766 us with every cell walked to the end first, 688 with
+// this, 718 with a thread a cell throughout.
+constexpr int kCrowd = 72;
 constexpr int kPool = 224;     // neighbours of a warp's cells at a time (about 130 at one cell per bin)
 // Threads (cells) per block of the passes; of the cooperative pass over the
 // grid by the law: the spring laws four warps at 72 registers, so that seven
