@@ -148,10 +148,11 @@ static __global__ void k_eorder_gather(const unsigned* __restrict__ off, unsigne
 // POL: some resident simulation carries polarity; spring-only engines use the
 // instance without the polarity law's terms.
 // TB: threads per block (64, 96 or 128; the autotuner's choice).
-// Resident threads an SM: 768 for the spring laws leave 80 registers.  With 896
-// (72 registers) ordinary ensembles gain 1 % (32 x 20,000 cells 215 against 218
-// us a step), and crowded cells on the general path lose 4 to 7 % to the form
-// before (8 x 5,000 cells at nine a bin 3.03 against 2.39 ms, 2.91 before).
+// CROWDED: many cells a bin.  Resident threads an SM for the spring laws: 896 (72
+// registers), where 768 (80) take 1 to 5 % longer on ordinary ensembles (8.7M
+// cells 2.49 against 2.38 ms a step); crowded cells on the general path want the
+// registers (8 x 5,000 cells at nine a bin 3.03 against 2.39 ms, 2.91 with the
+// form before the pool; 8 x 2,000 at thirty 11.15, 10.43 and 10.40).
 #define TECS_NO_ROW kNoRow
 #define TECS_LOAD(p) __ldg(p)
 #define TECS_ROW_SLOTS(N, lo, hi) row_slots<N>(off, lo, hi)
@@ -165,8 +166,8 @@ static __global__ void k_eorder_gather(const unsigned* __restrict__ off, unsigne
 #define TECS_CAPTURING false
 #define TECS_CAPTURE(c, jj)
 
-template <int PASS, bool POL, int TB>
-static __global__ void __launch_bounds__(TB, (POL ? 672 : 768) / TB) k_epass(EngArgs e) {
+template <int PASS, bool POL, bool CROWDED, int TB>
+static __global__ void __launch_bounds__(TB, (POL ? 672 : CROWDED ? 768 : 896) / TB) k_epass(EngArgs e) {
   constexpr int D = 3;
   __shared__ unsigned hsim[TB];
   const unsigned n = e.off[e.nb_total];
@@ -328,6 +329,7 @@ struct tecs_engine {
   float gdt = 0.f;
   unsigned gC = 0, gNB = 0;  // the extents the captured graph covers (cells, bins)
   bool gpol = false;         // the captured graph runs the polarity-capable pass
+  bool gcrowd = false;       // ... the pass for crowded bins
   int kernels = 7;
   unsigned pass_threads = 96;  // threads per block of the force passes (64, 96 or 128)
   unsigned gTB = 0;            // ... in the captured graph
@@ -416,11 +418,14 @@ int enqueue_engine_step(tecs_engine* e, float dt) {
 #define EPASS(T)                                                    \
   if (TB == T) {                                                    \
     if (e->gpol) {                                                  \
-      k_epass<1, true, T><<<blocks, T, 0, e->stream>>>(a1);         \
-      k_epass<2, true, T><<<blocks, T, 0, e->stream>>>(a2);         \
+      k_epass<1, true, false, T><<<blocks, T, 0, e->stream>>>(a1);  \
+      k_epass<2, true, false, T><<<blocks, T, 0, e->stream>>>(a2);  \
+    } else if (e->gcrowd) {                                         \
+      k_epass<1, false, true, T><<<blocks, T, 0, e->stream>>>(a1);  \
+      k_epass<2, false, true, T><<<blocks, T, 0, e->stream>>>(a2);  \
     } else {                                                        \
-      k_epass<1, false, T><<<blocks, T, 0, e->stream>>>(a1);        \
-      k_epass<2, false, T><<<blocks, T, 0, e->stream>>>(a2);        \
+      k_epass<1, false, false, T><<<blocks, T, 0, e->stream>>>(a1); \
+      k_epass<2, false, false, T><<<blocks, T, 0, e->stream>>>(a2); \
     }                                                               \
   }
   EPASS(64) EPASS(96) EPASS(128)
@@ -574,7 +579,7 @@ int tecs_engine_add(tecs_engine* e, const tecs_sim_desc* d, const float* positio
     g.mn[k] = d->min_bounds[k];
     g.ext[k] = (int)std::ceil((d->max_bounds[k] - d->min_bounds[k]) / g.bin_size);
     if (g.ext[k] < 1) return fail("max_bounds must exceed min_bounds");
-    if (g.ext[k] > 1023) return fail("the engine packs bin coordinates in 10 bits: extent <= 1023 bins");
+    if (g.ext[k] > 1023) return fail("the engine takes grids of at most 1023 bins a side");
     nb *= (unsigned long long)g.ext[k];
   }
   if (g.R != 1 || g.bin_size < d->cutoff) return fail("the engine needs bin_size_scale >= 1");
@@ -667,19 +672,25 @@ int tecs_engine_step(tecs_engine* e, double dt, int n_steps) {
       e->n_dirty = false;
     }
     unsigned hwm = 0;
+    double bins = 0.0;
     bool pol = false;
     for (unsigned k = 0; k < e->S; ++k)
       if (e->info[k].used) {
         hwm = std::max(hwm, e->info[k].bin_base + e->info[k].nbins);
+        bins += e->info[k].nbins;
         pol = pol || e->htable[k].has_pol;
       }
+    // (balls of tissue and their margins: at one cell a bin up to 0.5 a bin of the
+    // grid, packed tissue of 2.4 up to 1.1, 5,000 cells at nine 1.22)
+    const bool crowd = (double)e->n_resident > 1.2 * bins;
     const unsigned wantC = extent_class(e->n_resident, e->C), wantNB = extent_class(hwm, e->NB);
     if (!e->graph || e->gdt != fdt || wantC != e->gC || wantNB != e->gNB || pol != e->gpol ||
-        e->gTB != e->pass_threads) {
+        crowd != e->gcrowd || e->gTB != e->pass_threads) {
       if (e->graph) { cudaGraphExecDestroy(e->graph); e->graph = nullptr; }
       e->gC = wantC;
       e->gNB = wantNB;
       e->gpol = pol;
+      e->gcrowd = crowd;
       e->gTB = e->pass_threads;
       cudaGraph_t g;
       ECK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));

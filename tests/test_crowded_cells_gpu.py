@@ -155,3 +155,29 @@ def test_lone_cells_beside_a_clump(finder, dims, clump):
     s.take_step(0.001, 2)
     o.step(0.001, 2)
     np.testing.assert_array_equal(s.get_state()[0], o.get_state()[0])
+
+
+def test_engine_of_crowded_bins_runs_are_the_plain_ones():
+    # more than 1.2 resident cells a bin take another instance of the pass; a
+    # large sparse simulation that joins takes the engine back
+    xs = [cells(n, density, seed=8) for n, density in ((2000, 30.0), (1500, 20.0), (900, 0.2))]
+    settings = []
+    for x in xs:
+        mn, mx = wl.bounds_for(x)
+        settings.append(tg.Settings(agent_count=len(x), capacity=len(x),
+                                    pair_finder_settings=tg.PairFinderSettings(min_bounds=mn, max_bounds=mx)))
+    descs = [tg.make_desc(s, pair_finder=f, integrator="heun") for s, f in
+             zip(settings, ("binned_gabriel", "binned_all_pairs", "binned_gabriel"))]
+    bins = [bins_needed(d) for d in descs]
+    assert 3500 > 1.2 * sum(bins[:2]) and 4400 < 1.2 * sum(bins)
+    eng = Engine(cell_capacity=4400, bin_capacity=sum(bins) + 64, max_sims=4)
+    slots = [eng.add(d, x) for d, x in zip(descs[:2], xs)]
+    eng.step(1e-4, 2)
+    slots.append(eng.add(descs[2], xs[2]))
+    eng.step(1e-4, 2)
+    for x, st, f, slot, steps in zip(xs, settings, ("binned_gabriel", "binned_all_pairs", "binned_gabriel"), slots, (4, 4, 2)):
+        plain = tg.Simulation(st, pair_finder=f, integrator="heun")
+        plain.set_state(x)
+        plain.take_step(1e-4, steps)
+        np.testing.assert_array_equal(eng.download(slot)[0], plain.get_state()[0])
+    eng.close()
