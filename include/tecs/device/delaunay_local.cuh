@@ -29,11 +29,16 @@
 // sure that the circles, with the tolerance inside which delaunay_star.cuh looks for
 // further third points, lie within the gathered disk.
 //
+// The margins hold in any unit of length: they are shares of the cells' own
+// distances, each at least twice its rounding bound (tests/cpp/
+// delaunay_margins_host.cpp compares them with more bits).  A missed face cannot
+// pass: where some lines bound it, its tetrahedra are met from one third point
+// only, and where none does, every line has to be certain.
+//
 // What bounds it: instruction issue, then the latency of the few cells left to
 // the walk.  40k cells in space, one pass: 54 ms (the walk for every cell) ->
-// 2.0-2.4 (0.9 the first search, 0.5-0.8 the second over 7 % of the cells,
-// 0-0.8 the walk of at most 9 cells); 30k in the plane, two passes: 27-32 ->
-// 2.7-3.0 ms.
+// 1.7-2.1 (1.0 the first search, 0.6 the second over 7 % of the cells, 0-0.4 the
+// walk of a few cells); 30k in the plane, two passes: 27-42 -> 2.7-3.0 ms.
 #pragma once
 
 #include "delaunay_star.cuh"

@@ -624,7 +624,7 @@ constexpr unsigned kDelaunayNear = 64;  // points near i that each simplex is te
 // the lanes take the third points.
 // What bounds it: instruction issue (the spheres' arithmetic).  One thread per
 // third point that walks every l and every m in index order takes 400-660 ms
-// on 400 cells in 3-D, this form 1.4 ms.
+// on 400 cells in 3-D, this form 1.7 ms.
 template <int D>
 static __global__ void __launch_bounds__(kDelaunayThreads)
 k_delaunay_mult(const float4* __restrict__ X, const Counters* __restrict__ ctr, float rc2, unsigned stride,
@@ -1764,7 +1764,7 @@ static __global__ void __launch_bounds__(kCoopThreads<FORCE>, kCoopBlocks)
 // their reads and wait before their writes, a whole pass later.  A second
 // barrier ends a step, and the next one follows in the same launch.
 // The arithmetic is that of the passes over the grid: bit-identical runs.
-// 1000 cells, all-pairs: 25 -> 7.7 us a step (counts, scan, scatter and gather
+// 1000 cells, all-pairs: 25 -> 8.1 us a step (counts, scan, scatter and gather
 // through global memory between four cluster barriers, one launch a step: 21;
 // over the grid: 23).
 // The cluster size is set at launch (16 blocks: past the portable 8, opted
