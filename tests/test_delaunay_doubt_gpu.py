@@ -69,3 +69,11 @@ def test_a_few_cells(host_search, n, dims, cutoff):  # noqa: F811
     # walked all (up to six in space, eight in the plane) or searched first
     x = np.ascontiguousarray(wl.ball(n, 3)[:, :dims])
     assert found(x, cutoff) == expected(host_search, x, cutoff)
+
+
+@pytest.mark.parametrize("n", [511, 512, 513, 700])
+def test_sets_with_and_without_points_tested_first(host_search, n):  # noqa: F811
+    # every cell in cutoff: all are walked, in the plane with a list of points
+    # to test first past 512 cells
+    x = wl.disk(n, 4)
+    assert found(x, 1e3) == expected(host_search, x, 1e3)
